@@ -17,18 +17,21 @@ struct Box {
     R mn[3], mx[3];
 };
 
-// Padded AABB of segment k (k has hasNext).
+// Padded AABB of segment k (k has hasNext).  reach: the larger predicted displacement of its
+// endpoints (0 without the velocity radius), its share of a pair's filter distance.
 template <typename R>
-__device__ __forceinline__ Box<R> segment_box(const Dev<R>& d, int k, const SceneParams<R>& sp) {
+__device__ __forceinline__ Box<R> segment_box(const Dev<R>& d, int k, const SceneParams<R>& sp, R& reach) {
     typedef Ex<R> E;
     const V4<R> p0 = d.pos[k];
     const V4<R> p1 = d.pos[k + 1];
     R pad = sp.sdr;
+    reach = R(0);
     if (sp.useVelRadius) {
         const D2<R> dk = d.dx[0][k];
         const R l0 = xlen2(xyz(dk.a));
         const R l1 = xlen2(xyz(dk.b));
-        pad = E::add(pad, E::sqrt(ymax(l0, l1)));
+        reach = E::sqrt(ymax(l0, l1));
+        pad = E::add(pad, reach);
     }
     Box<R> b;
     b.mn[0] = E::sub(ymin(p0.x, p1.x), pad);
@@ -47,28 +50,58 @@ __device__ __forceinline__ bool box_overlap(const Box<R>& q, const R* mn, const 
            mn[2] <= q.mx[2];
 }
 
-// Narrow-phase decision for segments x < y (both with hasNext, same scene).
+// Narrow-phase decision for segments x < y (both with hasNext, same scene): not joined by a
+// connection, not neighbours on a yarn, and closer than the filter distance, to which each
+// segment adds its reach.
 template <typename R>
-__device__ __forceinline__ bool pair_keep(const Dev<R>& d, int x, int y, const SceneParams<R>& sp) {
-    typedef Ex<R> E;
+__device__ __forceinline__ bool pair_joined(const Dev<R>& d, int x, int y) {
     const int c0 = d.vp[x].cid;
     const int c1 = d.vp[x + 1].cid;
-    if (c0 == y || c1 == y || c0 == y + 1 || c1 == y + 1) return false;
-    if (y - x <= 2) return false;
+    return c0 == y || c1 == y || c0 == y + 1 || c1 == y + 1;
+}
+
+template <typename R>
+__device__ __forceinline__ R pair_distance2(const Dev<R>& d, int x, int y) {
     const V3<R> a0 = xyz(d.pos[x]);
     const V3<R> a1 = xsub(xyz(d.pos[x + 1]), a0);
     const V3<R> b0 = xsub(xyz(d.pos[y]), a0);
     const V3<R> b1 = xsub(xyz(d.pos[y + 1]), a0);
     const UVT<R> uv = closest_uv_exact(a1, b0, b1);
     const V3<R> nrm = xsub(xscale(uv.u, a1), xmix(b0, b1, uv.v));
-    const R d2 = xlen2(nrm);
+    return xlen2(nrm);
+}
+
+template <typename R>
+__device__ __forceinline__ bool pair_within(R d2, R reachX, R reachY, const SceneParams<R>& sp) {
+    typedef Ex<R> E;
     R r = E::mul(R(2), sp.sdr);
     if (sp.useVelRadius) {
-        const D2<R> dxx = d.dx[0][x], dxy = d.dx[0][y];
-        r = E::add(r, E::sqrt(ymax(xlen2(xyz(dxx.a)), xlen2(xyz(dxx.b)))));
-        r = E::add(r, E::sqrt(ymax(xlen2(xyz(dxy.a)), xlen2(xyz(dxy.b)))));
+        r = E::add(r, reachX);
+        r = E::add(r, reachY);
     }
     return d2 < E::mul(r, r);
+}
+
+template <typename R>
+__device__ __forceinline__ R segment_reach(const Dev<R>& d, int k) {
+    const D2<R> dk = d.dx[0][k];
+    return Ex<R>::sqrt(ymax(xlen2(xyz(dk.a)), xlen2(xyz(dk.b))));
+}
+
+template <typename R>
+__device__ __forceinline__ bool pair_keep(const Dev<R>& d, int x, int y, const SceneParams<R>& sp) {
+    if (pair_joined(d, x, y) || y - x <= 2) return false;
+    const R d2 = pair_distance2(d, x, y);
+    const bool vr = sp.useVelRadius != 0;
+    return pair_within(d2, vr ? segment_reach(d, x) : R(0), vr ? segment_reach(d, y) : R(0), sp);
+}
+
+// Appends y to x's contact list.  The count keeps growing past MAX_COLS so that the list
+// kernel can report the overflow (collision.cu:80-90).
+template <typename R>
+__device__ __forceinline__ void list_append(const Dev<R>& d, int x, int y) {
+    const int pos = atomicAdd(&d.numCols[x], 1);
+    if (pos < MAX_COLS) d.cols[col_at(x, pos)] = y;
 }
 
 // Step-size limit (collision.cu:121-159), split so that contacts can be spread over threads:

@@ -19,7 +19,7 @@
 //   csrCols  int    partner ids (sorted within each vertex's range)
 //   relA/B   V4,R2  partner endpoints relative to p0, staged per substep in the same slots
 //                   while the slot is below relCap (the one-block path stages rows of RELCAP)
-// Segments are the vertices with hasNext; segs[] lists them and is the leaf set of the BVH.
+// Segments are the vertices with hasNext; segs[] lists them, scene after scene.
 #pragma once
 #include "ybmath.cuh"
 
@@ -142,6 +142,18 @@ struct alignas(16) QRec {
     int k, sc;
 };
 
+// Clusters of a scene: runs of 32 segments in curve order, and the levels of 32 nodes each
+// above them.  Level 0 is the clusters; `top` is the first level with at most 32 nodes.
+constexpr int CURVE_AXIS = 13;              // bits per axis of the curve position
+constexpr int CURVE_BITS = 3 * CURVE_AXIS;  // ... and in all; the scene id is above them
+constexpr int CLUS_LEVELS = 4;              // 32^5 segments
+struct SceneClus {
+    int segBase, segCount;     // sorted positions of the scene's segments
+    int lvl[CLUS_LEVELS];      // first node of the scene in each level's arrays
+    int count[CLUS_LEVELS];    // nodes of the scene in each level
+    int top;
+};
+
 template <typename R>
 struct Dev {
     int n;            // vertices
@@ -182,9 +194,20 @@ struct Dev {
     int* sceneRoot;   // child code of each scene's subtree root (or INT_MIN when empty)
     int* sceneLast;   // sorted position of the last leaf of each scene's subtree
     unsigned* travNext;   // next query (sorted position) handed out by the traversal
-    int travBlocks[3];    // persistent traversal grid of each walk mode (travPacket)
-    int travPacket;       // 2: one walk per lane with warp-cooperative record loads (default),
-                          // 1: one walk per warp for 32 queries (k_traverse_packet), 0: one per lane
+    int travBlocks[2];    // persistent traversal grid of the BVH walks (travPacket 0, 1)
+    int travPacket;       // 2: cluster pairs (k_pairs, default), 1: one BVH walk per warp for 32
+                          // queries (k_traverse_packet), 0: one per lane (k_traverse)
+    // clusters of 32 segments in curve order (k_pairs.cu)
+    int nclus, nl1;       // clusters and level-1 nodes of all scenes
+    int pairWarps;        // fewest warps the pair search is spread over
+    float4 *leafLo, *leafHi;  // 32 per cluster: padded box of each segment; leafLo.w = its vertex
+                              // (-1: none), leafHi.w = its reach (segment_box)
+    int* sceneGlued;      // 1: some vertex of the scene has a connection
+    float4 *lvlLo[CLUS_LEVELS], *lvlHi[CLUS_LEVELS];
+    unsigned* lvlCount[CLUS_LEVELS];  // arrivals at the nodes of levels 2 and 3 (zero between launches)
+    SceneClus* sceneClus;
+    int* clusScene;       // scene of each cluster
+    int* l1Scene;         // scene of each level-1 node
     unsigned long long* keys[2];
     int* vals[2];
     unsigned* sceneBox;   // 6 ordered-uint per scene: min xyz, max xyz of segment midpoints
@@ -204,6 +227,10 @@ template <typename R> void launch_bvh_refit(const Dev<R>& d, cudaStream_t s);
 template <typename R> void launch_traverse(const Dev<R>& d, cudaStream_t s);  // + list sort + step limit (2 kernels)
 template <typename R> int traverse_blocks_per_sm(int mode);  // resident traversal blocks per SM (persistent grid)
 template <typename R> void launch_lists_step_limit(const Dev<R>& d, cudaStream_t s);  // step limit over segments
+// Segment, cluster and level boxes in curve order; the cluster-pair search; per-scene boxes.
+template <typename R> void launch_boxes(const Dev<R>& d, cudaStream_t s);
+template <typename R> void launch_pairs(const Dev<R>& d, cudaStream_t s);
+template <typename R> void launch_scene_box(const Dev<R>& d, float* out, cudaStream_t s);
 template <typename R> void launch_bvh_reset(const Dev<R>& d, cudaStream_t s);
 // Places driven vertices on their prescribed motion at the start of an advance of length dt.
 template <typename R>

@@ -1,4 +1,4 @@
-// io.cuh - launchers for layout conversion, diagnostics and BVH root boxes (k_io.cu).
+// io.cuh - launchers for layout conversion, diagnostics (k_io.cu).
 #pragma once
 #include "engine.cuh"
 
@@ -13,7 +13,6 @@ template <typename R> void launch_relayout(const Dev<R>& d, const int* sceneOf, 
 template <typename R> void launch_zero_vel(const Dev<R>& d, cudaStream_t s);
 template <typename R>
 void launch_state_f64(const Dev<R>& d, int buf, double* pos, double* vel, double* q, double* dx, cudaStream_t s);
-template <typename R> void launch_scene_root_box(const Dev<R>& d, float* out, cudaStream_t s);
 // Writes 8 doubles per block into part; returns the number of blocks.
 template <typename R> int launch_diag(const Dev<R>& d, double* part, cudaStream_t s);
 // Largest change of the Newton iterate made by the last iteration (which read buffer src and

@@ -1,18 +1,19 @@
-// k_bvh.cu - linear BVH over segment AABBs and the broadphase that emits contact lists.
+// k_bvh.cu - curve order of the segments, the linear BVH over their AABBs with its two walks, and
+// the list pass.
 //
 // The reference calls an LBVH library whose source is not part of the reference project
-// (KittenEngine/KittenGpuLBVH is an empty submodule; call sites collision.cu:94-119).  This
-// is a new implementation of the published method:
-//   * leaf keys: 30-bit Morton code of the segment midpoint, normalised by its scene's
-//     bounds, with the scene id above bit 30 so that every scene is one subtree;
-//   * stable LSD radix sort of (key, segment) pairs (k_sort.cu);
+// (KittenEngine/KittenGpuLBVH is an empty submodule; call sites collision.cu:94-119).
+//   * keys: position of the segment's midpoint along a Hilbert curve over its scene's bounding
+//     cube, with the scene id above it so that every scene is one range;
+//   * stable LSD radix sort of (key, segment) pairs (k_sort.cu).
+// The default broadphase (k_pairs.cu) needs only this order.  The BVH walks (yb_set_traversal
+// 0 and 1) build on it:
 //   * Karras 2012 binary radix tree emission, one thread per internal node, ties between
 //     equal keys broken by leaf position;
 //   * bottom-up AABB refit with one atomic arrival counter per internal node;
 //   * traversal: every segment walks its own scene's subtree with its own padded box and
-//     keeps the partners that pass the narrow-phase filter (detect.cuh).  Each segment
-//     writes only its own list (no atomics on other segments' lists); the list is then
-//     sorted by partner id and the step-size limit is computed from it in the same thread.
+//     keeps the partners that pass the narrow-phase filter (detect.cuh).
+// All of them append kept pairs to both segments' lists, which the list pass then sorts.
 #include <cuda/atomic>
 
 #include "detect.cuh"
@@ -72,8 +73,41 @@ __global__ void __launch_bounds__(256) k_scene_bounds(Dev<R> d) {
     }
 }
 
+// Position of cell (x, y, z) along the Hilbert curve of CURVE_AXIS bits per axis (J. Skilling,
+// "Programming the Hilbert curve", 2004: undo the excess work bit by bit, Gray encode, then
+// interleave with x most significant).
+__device__ __forceinline__ unsigned long long hilbert_index(unsigned x, unsigned y, unsigned z) {
+    unsigned X[3] = {x, y, z};
+    for (unsigned q = 1u << (CURVE_AXIS - 1); q > 1; q >>= 1) {
+        const unsigned p = q - 1;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            if (X[a] & q) {
+                X[0] ^= p;
+            } else {
+                const unsigned t = (X[0] ^ X[a]) & p;
+                X[0] ^= t;
+                X[a] ^= t;
+            }
+        }
+    }
+    X[1] ^= X[0];
+    X[2] ^= X[1];
+    unsigned t = 0;
+    for (unsigned q = 1u << (CURVE_AXIS - 1); q > 1; q >>= 1)
+        if (X[2] & q) t ^= q - 1;
+    unsigned long long key = 0;
+    for (int b = CURVE_AXIS - 1; b >= 0; b--)
+#pragma unroll
+        for (int a = 0; a < 3; a++) key = (key << 1) | (((X[a] ^ t) >> b) & 1u);
+    return key;
+}
+
+// Sort keys.  The cells are cubes (the scene's largest extent over 2^CURVE_AXIS): boxes are
+// padded by the same distance along every axis, so runs of the curve should be as short along
+// each.
 template <typename R>
-__global__ void __launch_bounds__(256) k_morton(Dev<R> d) {
+__global__ void __launch_bounds__(256) k_curve_keys(Dev<R> d) {
     const int si = blockIdx.x * blockDim.x + threadIdx.x;
     if (si >= d.nseg) return;
     const int k = d.segs[si];
@@ -81,18 +115,21 @@ __global__ void __launch_bounds__(256) k_morton(Dev<R> d) {
     const V4<R> p0 = d.pos[k], p1 = d.pos[k + 1];
     const float m[3] = {(float)((p0.x + p1.x) * R(0.5)), (float)((p0.y + p1.y) * R(0.5)),
                         (float)((p0.z + p1.z) * R(0.5))};
-    uint32_t code = 0;
+    float lo[3], ext = 0.f;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float lo = ord2f(d.sceneBox[6 * sc + a]);
-        const float hi = ord2f(d.sceneBox[6 * sc + 3 + a]);
-        const float ext = hi - lo;
-        float c = ext > 0.f ? (m[a] - lo) / ext : 0.5f;
-        int qv = (int)(c * 1024.f);
-        qv = qv < 0 ? 0 : (qv > 1023 ? 1023 : qv);
-        code |= morton_spread10((uint32_t)qv) << (2 - a);
+        lo[a] = ord2f(d.sceneBox[6 * sc + a]);
+        ext = fmaxf(ext, ord2f(d.sceneBox[6 * sc + 3 + a]) - lo[a]);
     }
-    d.keys[0][si] = ((unsigned long long)sc << 30) | code;
+    unsigned cell[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        constexpr int N = 1 << CURVE_AXIS;
+        const float c = ext > 0.f ? (m[a] - lo[a]) / ext : 0.5f;
+        const int q = (int)(c * (float)N);
+        cell[a] = (unsigned)(q < 0 ? 0 : (q > N - 1 ? N - 1 : q));
+    }
+    d.keys[0][si] = ((unsigned long long)sc << CURVE_BITS) | hilbert_index(cell[0], cell[1], cell[2]);
     d.vals[0][si] = k;
 }
 
@@ -112,9 +149,9 @@ __global__ void __launch_bounds__(256) k_karras(Dev<R> d, const unsigned long lo
     if (i >= n) return;
     // single-leaf scenes
     {
-        const unsigned long long sc = keys[i] >> 30;
-        const bool lo = (i == 0) || ((keys[i - 1] >> 30) != sc);
-        const bool hi = (i == n - 1) || ((keys[i + 1] >> 30) != sc);
+        const unsigned long long sc = keys[i] >> CURVE_BITS;
+        const bool lo = (i == 0) || ((keys[i - 1] >> CURVE_BITS) != sc);
+        const bool hi = (i == n - 1) || ((keys[i + 1] >> CURVE_BITS) != sc);
         if (lo && hi) d.sceneRoot[sc] = -(vals[i] + 1);
     }
     if (i >= n - 1) return;
@@ -153,9 +190,9 @@ __global__ void __launch_bounds__(256) k_karras(Dev<R> d, const unsigned long lo
         d.nodes[gamma + 1].parent = i;
     }
     if (i == 0) nd.parent = -1;
-    const unsigned long long sc = keys[first] >> 30;
-    if ((keys[last] >> 30) == sc && (first == 0 || (keys[first - 1] >> 30) != sc) &&
-        (last == n - 1 || (keys[last + 1] >> 30) != sc)) {
+    const unsigned long long sc = keys[first] >> CURVE_BITS;
+    if ((keys[last] >> CURVE_BITS) == sc && (first == 0 || (keys[first - 1] >> CURVE_BITS) != sc) &&
+        (last == n - 1 || (keys[last + 1] >> CURVE_BITS) != sc)) {
         d.sceneRoot[sc] = i;
         d.sceneLast[sc] = last;
     }
@@ -181,7 +218,8 @@ __global__ void __launch_bounds__(256) k_refit(Dev<R> d, const int* __restrict__
     const int k = sortedVals[p];
     const int sc = scene_of(d.vp[k].flags);
     const SceneParams<R>& sp = d.sp[sc];
-    Box<R> b = segment_box(d, k, sp);
+    R reach;
+    Box<R> b = segment_box(d, k, sp, reach);
     {
         QRec<R> r;
 #pragma unroll
@@ -260,7 +298,7 @@ __global__ void __launch_bounds__(256) k_depth_mark(Dev<R> d, int fin) {
     if (i >= d.nseg - 1) return;
     if (d.depJump[fin][i] >= 0) *d.wideAll = 1;
     // internal node i's leaf range has leaf i at one end, so leaf i's key names its scene
-    const int root = d.sceneRoot[(int)(d.keys[0][i] >> 30)];
+    const int root = d.sceneRoot[(int)(d.keys[0][i] >> CURVE_BITS)];
     int used = 0;
     if (root >= 0) {
         const int rel = d.depDist[fin][i] - d.depDist[fin][root];
@@ -318,14 +356,6 @@ constexpr int TRAV_WARPS = TRAV_THREADS / 32;
 constexpr int TRAV_QCAP = 160;      // < 32 left over + up to 4 candidates per lane
 constexpr int TRAV_GRAB = 32;       // queries a warp takes from the counter at a time
 
-// Appends y to x's contact list.  The count keeps growing past MAX_COLS so that the list
-// kernel can report the overflow (collision.cu:80-90).
-template <typename R>
-__device__ __forceinline__ void list_append(const Dev<R>& d, int x, int y) {
-    const int pos = atomicAdd(&d.numCols[x], 1);
-    if (pos < MAX_COLS) d.cols[col_at(x, pos)] = y;
-}
-
 // Broadphase + narrow phase.  Every segment queries the tree once with its own box (the
 // sorted leaves of the last rebuild, taken in Morton order, so neighbouring lanes start on
 // neighbouring queries).  Each unordered pair is found by exactly one of its two segments:
@@ -352,47 +382,10 @@ __device__ __forceinline__ void trav_load_wide(const WNode<R>* wide, int node, W
     }
 }
 
-// Warp-cooperative load of the 32 lanes' current records (FP32 records: eight 16-byte
-// pieces, one 128-byte line).  Loading its own record, each lane would touch 32 different lines
-// with each of its 8 loads (256 L1 wavefronts per step of the warp); here load r fetches piece
-// (lane & 7) of the record of lane 4r + (lane >> 3), so each load covers 4 whole lines (32
-// wavefronts per step), and the pieces reach their lanes through shared memory (rows padded to
-// 9 pieces, so the reads back are free of bank conflicts).  node < 0: the lane loads nothing.
-constexpr int COOP_ROW = 9;
-
-__device__ __forceinline__ void coop_load_wide(const WNode<float>* wide, int node, float4 (*rows)[COOP_ROW], int lane) {
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const int owner = 4 * r + (lane >> 3);
-        const int on = __shfl_sync(0xffffffffu, node, owner);
-        if (on >= 0) rows[owner][lane & 7] = __ldg(reinterpret_cast<const float4*>(wide + on) + (lane & 7));
-    }
-    __syncwarp();
-}
-
-// Entry e of a wide record: from the lane's shared-memory row (cooperative load) or from
-// the record in registers.
 template <typename R>
-__device__ __forceinline__ WEntry<R> wide_entry(const WNode<R>& w, const float4* row, int e, bool fromRow) {
-    if constexpr (sizeof(R) == 4) {
-        if (fromRow) {
-            const float4 A = row[2 * e], B = row[2 * e + 1];  // (mn xyz, mx x), (mx yz, code, last)
-            WEntry<R> x;
-            x.mn[0] = A.x; x.mn[1] = A.y; x.mn[2] = A.z;
-            x.mx[0] = A.w; x.mx[1] = B.x; x.mx[2] = B.y;
-            x.code = __float_as_int(B.z);
-            x.last = __float_as_int(B.w);
-            return x;
-        }
-    }
-    return w.e[e];
-}
-
-template <typename R, bool COOP>
 __global__ void __launch_bounds__(TRAV_THREADS) k_traverse(Dev<R> d) {
     __shared__ int sQx[TRAV_WARPS][TRAV_QCAP];
     __shared__ int sQy[TRAV_WARPS][TRAV_QCAP];
-    __shared__ float4 sRec[COOP ? TRAV_WARPS : 1][COOP ? 32 : 1][COOP_ROW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int nseg = d.nseg;
@@ -463,15 +456,13 @@ __global__ void __launch_bounds__(TRAV_THREADS) k_traverse(Dev<R> d) {
             atomicOr(&d.err[EW_INTERNAL], IE_BVH_STACK);
             walking = false;
         }
-        constexpr bool ROW = COOP && sizeof(R) == 4;
-        WNode<R> w;
-        if constexpr (ROW) coop_load_wide(d.wide, walking ? node : -1, sRec[warp], lane);
         if (walking) {
-            if constexpr (!ROW) trav_load_wide(d.wide, node, w);
+            WNode<R> w;
+            trav_load_wide(d.wide, node, w);
             int next = -1;
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const WEntry<R> x = wide_entry(w, sRec[COOP ? warp : 0][COOP ? lane : 0], e, ROW);
+                const WEntry<R>& x = w.e[e];
                 const bool hit = x.last > qi && qb.mn[0] <= x.mx[0] && x.mn[0] <= qb.mx[0] && qb.mn[1] <= x.mx[1] &&
                                  x.mn[1] <= qb.mx[1] && qb.mn[2] <= x.mx[2] && x.mn[2] <= qb.mx[2];
                 if (!hit) continue;
@@ -510,7 +501,7 @@ __global__ void __launch_bounds__(TRAV_THREADS) k_traverse(Dev<R> d) {
             }
         }
         qn += __shfl_sync(0xffffffffu, incl, 31);
-        __syncwarp();  // also: every lane has read its record row before the next load fills it
+        __syncwarp();
         const bool drain = !more && !__any_sync(0xffffffffu, walking);
         while (qn >= 32 || (drain && qn > 0)) {
             const int m = min(qn, 32);
@@ -934,22 +925,24 @@ void launch_bvh_rebuild(const Dev<R>& d, cudaStream_t s, void* sortScratch, size
     const int nb = (d.nseg + 255) / 256;
     k_scene_box_init<R><<<(d.numScenes + 127) / 128, 128, 0, s>>>(d);
     k_scene_bounds<R><<<nb, 256, 0, s>>>(d);
-    k_morton<R><<<nb, 256, 0, s>>>(d);
+    k_curve_keys<R><<<nb, 256, 0, s>>>(d);
     unsigned long long* keys[2] = {d.keys[0], d.keys[1]};
     int* vals[2] = {d.vals[0], d.vals[1]};
     const int buf = radix_sort_pairs(keys, vals, d.nseg, keyBits, sortScratch, d.err + EW_INTERNAL, s);
-    // After sorting, buffer 0 must hold the sorted pairs (refit/karras read it).
+    // After sorting, buffer 0 must hold the sorted pairs (boxes/refit/karras read it).
     if (buf != 0) {
         cudaMemcpyAsync(d.keys[0], d.keys[1], sizeof(unsigned long long) * d.nseg, cudaMemcpyDeviceToDevice, s);
         cudaMemcpyAsync(d.vals[0], d.vals[1], sizeof(int) * d.nseg, cudaMemcpyDeviceToDevice, s);
     }
-    k_karras<R><<<nb, 256, 0, s>>>(d, d.keys[0], d.vals[0]);
-    // DEPTH_LAUNCHES kernels: which wide records the walk can load
-    const int ib = (max(d.nseg - 1, 1) + 255) / 256;
-    cudaMemsetAsync(d.wideAll, 0, sizeof(int), s);
-    k_depth_init<R><<<ib, 256, 0, s>>>(d);
-    for (int r = 0; r < DEPTH_ROUNDS; r++) k_depth_jump<R><<<ib, 256, 0, s>>>(d, r & 1);
-    k_depth_mark<R><<<ib, 256, 0, s>>>(d, DEPTH_ROUNDS & 1);
+    if (d.travPacket != 2) {
+        k_karras<R><<<nb, 256, 0, s>>>(d, d.keys[0], d.vals[0]);
+        // DEPTH_LAUNCHES kernels: which wide records the walk can load
+        const int ib = (max(d.nseg - 1, 1) + 255) / 256;
+        cudaMemsetAsync(d.wideAll, 0, sizeof(int), s);
+        k_depth_init<R><<<ib, 256, 0, s>>>(d);
+        for (int r = 0; r < DEPTH_ROUNDS; r++) k_depth_jump<R><<<ib, 256, 0, s>>>(d, r & 1);
+        k_depth_mark<R><<<ib, 256, 0, s>>>(d, DEPTH_ROUNDS & 1);
+    }
     launch_bvh_refit(d, s);
 }
 
@@ -960,7 +953,10 @@ void launch_bvh_reset(const Dev<R>& d, cudaStream_t s) {
 
 template <typename R>
 void launch_bvh_refit(const Dev<R>& d, cudaStream_t s) {
-    if (d.nseg <= 0) return;  // one segment: no internal node, but its query record is written
+    if (d.nseg <= 0) return;
+    launch_boxes(d, s);  // also for bounds()
+    if (d.travPacket == 2) return;
+    // one segment: no internal node, but its query record is written
     if (d.nseg > 1) cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * (d.nseg - 1), s);
     k_refit<R><<<(d.nseg + 255) / 256, 256, 0, s>>>(d, d.vals[0]);
     k_widen<R><<<(d.nseg + 255) / 256, 256, 0, s>>>(d);  // at least one block; the kernel bounds itself
@@ -977,14 +973,16 @@ template <typename R>
 void launch_traverse(const Dev<R>& d, cudaStream_t s) {
     if (d.nseg <= 0) return;
     cudaMemsetAsync(d.numCols, 0, sizeof(int) * d.n, s);
-    cudaMemsetAsync(d.travNext, 0, sizeof(unsigned), s);
-    const int blocks = min((d.nseg + TRAV_THREADS - 1) / TRAV_THREADS, max(d.travBlocks[d.travPacket], 1));
-    if (d.travPacket == 1)
-        k_traverse_packet<R><<<blocks, TRAV_THREADS, 0, s>>>(d);
-    else if (d.travPacket == 2)
-        k_traverse<R, true><<<blocks, TRAV_THREADS, 0, s>>>(d);
-    else
-        k_traverse<R, false><<<blocks, TRAV_THREADS, 0, s>>>(d);
+    if (d.travPacket == 2) {
+        launch_pairs(d, s);
+    } else {
+        cudaMemsetAsync(d.travNext, 0, sizeof(unsigned), s);
+        const int blocks = min((d.nseg + TRAV_THREADS - 1) / TRAV_THREADS, max(d.travBlocks[d.travPacket], 1));
+        if (d.travPacket == 1)
+            k_traverse_packet<R><<<blocks, TRAV_THREADS, 0, s>>>(d);
+        else
+            k_traverse<R><<<blocks, TRAV_THREADS, 0, s>>>(d);
+    }
     launch_lists(d, 1, s);
 }
 
@@ -1008,8 +1006,7 @@ int traverse_blocks_per_sm(int mode) {  // resident blocks of the traversal kern
     int b = 0;
     const cudaError_t e =
         mode == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traverse_packet<R>, TRAV_THREADS, 0)
-        : mode == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traverse<R, true>, TRAV_THREADS, 0)
-                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traverse<R, false>, TRAV_THREADS, 0);
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traverse<R>, TRAV_THREADS, 0);
     if (e != cudaSuccess || b < 1) {
         cudaGetLastError();
         return 4;

@@ -1,10 +1,9 @@
 // k_io.cu - host<->device layout conversion (AoS host arrays <-> SoA device state),
-// velocity reset, BVH root boxes and the FP64 diagnostic reductions.
+// velocity reset and the FP64 diagnostic reductions.
 //
 //   upload/copyTempData  KittenEngine/YarnBall/YarnBall.cu:239-254
 //   download             KittenEngine/YarnBall/YarnBall.cu:256-261
 //   zeroVels             KittenEngine/YarnBall/YarnBall.cu:263-274
-//   bounds               KittenEngine/YarnBall/YarnBall.cu:87-89
 #include "detect.cuh"
 #include "io.cuh"
 
@@ -36,6 +35,7 @@ __global__ void k_convert_in(Dev<R> d, const HostVertex* __restrict__ hv, const 
     if (i == 0 || sceneOf[i - 1] != sceneOf[i]) fl &= ~(uint32_t)F_HAS_PREV;
     vp.flags = fl | ((uint32_t)sceneOf[i] << 8);
     d.vp[i] = vp;
+    if (vp.cid >= 0) d.sceneGlued[sceneOf[i]] = 1;
     V4<R> vel; vel.x = hvel[3 * i]; vel.y = hvel[3 * i + 1]; vel.z = hvel[3 * i + 2]; vel.w = R(0);
     d.vel[i] = vel;
     V4<R> q; q.x = hq[4 * i]; q.y = hq[4 * i + 1]; q.z = hq[4 * i + 2]; q.w = hq[4 * i + 3];
@@ -75,7 +75,10 @@ __global__ void k_relayout(Dev<R> d, const int* __restrict__ sceneOf, const int*
     if (i == d.n - 1 || sceneOf[i + 1] != sc) fl &= ~(uint32_t)(F_HAS_NEXT | F_HAS_NEXT_ORI);
     if (i == 0 || sceneOf[i - 1] != sc) fl &= ~(uint32_t)F_HAS_PREV;
     vp.flags = fl | ((uint32_t)sc << 8);
-    if (vp.cid >= 0) vp.cid += delta[sc];
+    if (vp.cid >= 0) {
+        vp.cid += delta[sc];
+        d.sceneGlued[sc] = 1;
+    }
     d.vp[i] = vp;
 }
 
@@ -133,27 +136,6 @@ __global__ void k_state_f64(Dev<R> d, int buf, double* pos, double* vel, double*
     if (vel) { const V4<R> v = d.vel[i]; vel[3 * i] = v.x; vel[3 * i + 1] = v.y; vel[3 * i + 2] = v.z; }
     if (q) { const V4<R> a = d.q[buf][i]; q[4 * i] = a.x; q[4 * i + 1] = a.y; q[4 * i + 2] = a.z; q[4 * i + 3] = a.w; }
     if (dx) { const V4<R> a = d.dx[buf][i].a; dx[4 * i] = a.x; dx[4 * i + 1] = a.y; dx[4 * i + 2] = a.z; dx[4 * i + 3] = a.w; }
-}
-
-// Root box of each scene's subtree (refit must have run).
-template <typename R>
-__global__ void k_scene_root_box(Dev<R> d, float* out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.numScenes) return;
-    const int r = d.sceneRoot[s];
-    float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    if (r >= 0) {
-        const BNode<R>& nd = d.nodes[r];
-        for (int a = 0; a < 3; a++) {
-            b[a] = (float)ymin(nd.lmin[a], nd.rmin[a]);
-            b[3 + a] = (float)ymax(nd.lmax[a], nd.rmax[a]);
-        }
-    } else if (r != INT_MIN) {
-        const int k = -r - 1;
-        const Box<R> bx = segment_box(d, k, d.sp[s]);
-        for (int a = 0; a < 3; a++) { b[a] = (float)bx.mn[a]; b[3 + a] = (float)bx.mx[a]; }
-    }
-    for (int a = 0; a < 6; a++) out[6 * s + a] = b[a];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -272,10 +254,6 @@ void launch_state_f64(const Dev<R>& d, int buf, double* pos, double* vel, double
     k_state_f64<R><<<(d.n + 255) / 256, 256, 0, s>>>(d, buf, pos, vel, q, dx);
 }
 template <typename R>
-void launch_scene_root_box(const Dev<R>& d, float* out, cudaStream_t s) {
-    k_scene_root_box<R><<<(d.numScenes + 127) / 128, 128, 0, s>>>(d, out);
-}
-template <typename R>
 int launch_diag(const Dev<R>& d, double* part, cudaStream_t s) {
     const int nb = (d.n + 255) / 256;
     if (nb > 0) k_diag<R><<<nb, 256, 0, s>>>(d, part);
@@ -310,7 +288,6 @@ void launch_iter_delta(const Dev<R>& d, int src, unsigned long long* slot, cudaS
                                       cudaStream_t);                                                         \
     template void launch_zero_vel<R>(const Dev<R>&, cudaStream_t);                                           \
     template void launch_state_f64<R>(const Dev<R>&, int, double*, double*, double*, double*, cudaStream_t); \
-    template void launch_scene_root_box<R>(const Dev<R>&, float*, cudaStream_t);                             \
     template void launch_iter_delta<R>(const Dev<R>&, int, unsigned long long*, cudaStream_t);               \
     template int launch_diag<R>(const Dev<R>&, double*, cudaStream_t);
 YB_INST(float)

@@ -95,7 +95,7 @@ struct yb_sim {
     int iterLanes = 0;
     int iterPipe = 0;
     int useGraphs = 1;
-    int travPacket = 2;  // broadphase walk: 2 per query with cooperative loads, 1 per warp of 32 queries, 0 per query
+    int travPacket = 2;  // broadphase: 2 cluster pairs, 1 BVH walk per warp of 32 queries, 0 per query
     int useSmall = 1;    // advance small simulations with the one-block kernel
     uint64_t launches = 0;
     cudaStream_t stream = nullptr;     // active stream (own or the caller's)
@@ -310,7 +310,7 @@ struct Engine : EngineBase {
     cudaGraphExec_t graphs[GRAPH_TYPES] = {nullptr, nullptr, nullptr};
     uint64_t graphLaunches[GRAPH_TYPES] = {0, 0, 0};
     int graphItr = -1, graphThreads = -1, graphLanes = -1, graphPipe = -1, graphNseg = -1;
-    int keyBits = 30;
+    int keyBits = CURVE_BITS;
     int64_t penTotal = 0;
     float minDist = INFINITY;
 
@@ -374,6 +374,20 @@ struct Engine : EngineBase {
         want((void**)&d.sceneRoot, sizeof(int) * ns);
         want((void**)&d.sceneLast, sizeof(int) * ns);
         want((void**)&d.travNext, sizeof(unsigned) * 4);
+        // clusters: the last one of a scene may be partly filled, and so may the last node of a level
+        size_t nodesCap[CLUS_LEVELS];
+        for (int l = 0; l < CLUS_LEVELS; l++) nodesCap[l] = (l ? nodesCap[l - 1] : n) / 32 + ns;
+        want((void**)&d.sceneGlued, sizeof(int) * ns);
+        want((void**)&d.leafLo, sizeof(float4) * 32 * nodesCap[0]);
+        want((void**)&d.leafHi, sizeof(float4) * 32 * nodesCap[0]);
+        for (int l = 0; l < CLUS_LEVELS; l++) {
+            want((void**)&d.lvlLo[l], sizeof(float4) * nodesCap[l]);
+            want((void**)&d.lvlHi[l], sizeof(float4) * nodesCap[l]);
+            want((void**)&d.lvlCount[l], sizeof(unsigned) * nodesCap[l]);
+        }
+        want((void**)&d.sceneClus, sizeof(SceneClus) * ns);
+        want((void**)&d.clusScene, sizeof(int) * nodesCap[0]);
+        want((void**)&d.l1Scene, sizeof(int) * nodesCap[1]);
         want((void**)&d.keys[0], sizeof(unsigned long long) * n);
         want((void**)&d.keys[1], sizeof(unsigned long long) * n);
         want((void**)&d.vals[0], sizeof(int) * n);
@@ -403,7 +417,8 @@ struct Engine : EngineBase {
             int dev = 0, sms = 148;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            for (int m = 0; m < 3; m++) d.travBlocks[m] = sms * traverse_blocks_per_sm<R>(m);
+            for (int m = 0; m < 2; m++) d.travBlocks[m] = sms * traverse_blocks_per_sm<R>(m);
+            d.pairWarps = sms * 32;
         }
         d.travPacket = S->travPacket;
         YB_CUDA(cudaHostAlloc((void**)&spHost, sizeof(SceneParams<R>) * ns, cudaHostAllocDefault));
@@ -416,6 +431,8 @@ struct Engine : EngineBase {
         YB_CUDA(cudaMemsetAsync(d.csrOff, 0, sizeof(unsigned) * (n + 1), S->stream));
         YB_CUDA(cudaMemsetAsync(d.lastVel, 0, sizeof(V4<R>) * n, S->stream));
         YB_CUDA(cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * nn, S->stream));
+        for (int l = 0; l < CLUS_LEVELS; l++)
+            YB_CUDA(cudaMemsetAsync(d.lvlCount[l], 0, sizeof(unsigned) * nodesCap[l], S->stream));
         // records never built read as empty (last = 0 prunes every entry); until the first
         // rebuild marks the nodes, every record is built
         YB_CUDA(cudaMemsetAsync(d.wide, 0, sizeof(WNode<R>) * nn, S->stream));
@@ -436,9 +453,51 @@ struct Engine : EngineBase {
             for (int i = S->sceneOff[s]; i < S->sceneOff[s + 1]; i++) so[i] = s;
         d.n = S->n;
         d.numScenes = S->numScenes;
-        keyBits = 30 + scene_bits(S->numScenes);
+        keyBits = CURVE_BITS + scene_bits(S->numScenes);
         cudaError_t e = cudaMemcpyAsync(sceneOf, so.data(), sizeof(int) * so.size(), cudaMemcpyHostToDevice, S->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(S->stream);
+        return e;
+    }
+
+    // Clusters of 32 segments per scene and the levels above them, from S->segs (scene after
+    // scene, the order the sorted segments keep).  The copies read the vectors below until the
+    // caller synchronises.
+    std::vector<SceneClus> hostClus;
+    std::vector<int> hostClusScene, hostL1Scene;
+    cudaError_t upload_clusters() {
+        hostClus.assign((size_t)S->numScenes, SceneClus());
+        hostClusScene.clear();
+        hostL1Scene.clear();
+        int total[CLUS_LEVELS] = {};
+        auto at = S->segs.begin();
+        for (int s = 0; s < S->numScenes; s++) {
+            SceneClus& c = hostClus[s];
+            const auto end = std::lower_bound(at, S->segs.end(), S->sceneOff[s + 1]);
+            c.segBase = (int)(at - S->segs.begin());
+            c.segCount = (int)(end - at);
+            at = end;
+            int m = c.segCount;
+            for (int l = 0; l < CLUS_LEVELS; l++) {
+                m = (m + 31) / 32;
+                c.lvl[l] = total[l];
+                c.count[l] = m;
+                total[l] += m;
+            }
+            while (c.count[c.top] > 32) c.top++;
+            hostClusScene.resize((size_t)total[0], s);
+            hostL1Scene.resize((size_t)total[1], s);
+        }
+        d.nclus = total[0];
+        d.nl1 = total[1];
+        bvhBuilt = false;
+        cudaError_t e = cudaMemcpyAsync(d.sceneClus, hostClus.data(), sizeof(SceneClus) * hostClus.size(),
+                                        cudaMemcpyHostToDevice, S->stream);
+        if (e == cudaSuccess && total[0])
+            e = cudaMemcpyAsync(d.clusScene, hostClusScene.data(), sizeof(int) * hostClusScene.size(),
+                                cudaMemcpyHostToDevice, S->stream);
+        if (e == cudaSuccess && total[1])
+            e = cudaMemcpyAsync(d.l1Scene, hostL1Scene.data(), sizeof(int) * hostL1Scene.size(), cudaMemcpyHostToDevice,
+                                S->stream);
         return e;
     }
 
@@ -511,6 +570,8 @@ struct Engine : EngineBase {
     }
 
     yb_status load_device(FILE* f) override {
+        // any scene may hold connections (a non-zero flag only makes the filter look)
+        YB_CUDA(cudaMemset(d.sceneGlued, 1, sizeof(int) * (size_t)S->numScenes));
         for (auto& a : state_arrays()) {
             std::vector<char> h(a.second);
             if (fread(h.data(), 1, a.second, f) != a.second) return YB_ERR_INVALID_ARGUMENT;
@@ -550,6 +611,8 @@ struct Engine : EngineBase {
         YB_CUDA(cudaStreamSynchronize(S->stream));
         d.nseg = (int)segs.size();
         S->segs.swap(segs);
+        YB_CUDA(upload_clusters());
+        YB_CUDA(cudaStreamSynchronize(S->stream));
         S->lastBVHRebuild = INFINITY;
         invalidate_graphs();
         return YB_OK;
@@ -597,6 +660,7 @@ struct Engine : EngineBase {
             YB_CUDA(cudaMemcpyAsync(d.vp + to, sd.vp + so, sizeof(VP<R>) * m, cudaMemcpyDeviceToDevice, st));
         }
         YB_CUDA(cudaMemcpyAsync(sceneDelta, delta.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
+        YB_CUDA(cudaMemsetAsync(d.sceneGlued, 0, sizeof(int) * (size_t)S->numScenes, st));
         launch_relayout(d, sceneOf, sceneDelta, st);
         S->launches++;
         YB_CUDA(cudaMemsetAsync(d.numCols, 0, sizeof(int) * (size_t)S->n, st));
@@ -628,6 +692,8 @@ struct Engine : EngineBase {
         }
         if (changed && !S->segs.empty())
             YB_CUDA(cudaMemcpyAsync(d.segs, S->segs.data(), sizeof(int) * S->segs.size(), cudaMemcpyHostToDevice, st));
+        if (changed) YB_CUDA(upload_clusters());
+        YB_CUDA(cudaMemsetAsync(d.sceneGlued, 0, sizeof(int) * (size_t)S->numScenes, st));
         launch_convert_in(d, sv, (const float*)svel, (const float*)sq, (const float*)sqr, sceneOf, st);
         S->launches++;
         YB_CUDA(cudaGetLastError());
@@ -723,7 +789,13 @@ struct Engine : EngineBase {
     // Newton iterations per substep: shared by every scene (validate_all_meta).
     int num_itr() const { return (int)S->meta[0].numItr; }
 
-    // Enqueues one substep on the stream; returns the number of kernels it launches.
+    // Kernels of a rebuild and of a refit, with the boxes of either.
+    uint64_t refit_launches() const { return d.travPacket == 2 ? 1 : 3; }
+    uint64_t rebuild_launches() const {
+        const int passes = d.nseg > 1 ? (keyBits + 7) / 8 : 0;
+        return 3 + (d.nseg > 1 ? 2 + passes : 0) + (d.travPacket == 2 ? 0 : 1 + DEPTH_LAUNCHES) + refit_launches();
+    }
+
     // One substep's kernels on S->stream; returns how many were launched.  With slots, the
     // largest iterate change of Newton iteration it is reduced into slots[it] after it.
     uint64_t enqueue_substep(bool detect, bool rebuild, unsigned long long* slots = nullptr) override {
@@ -734,11 +806,10 @@ struct Engine : EngineBase {
             if (rebuild) {  // the schedule rebuilds first after any path that did not use the tree
                 launch_bvh_rebuild(d, st, sortScratch, sortBytes, keyBits);
                 bvhBuilt = true;
-                const int passes = d.nseg > 1 ? (keyBits + 7) / 8 : 0;
-                k += 3 + (d.nseg > 1 ? 2 + passes : 0) + 1 + DEPTH_LAUNCHES + 2;
+                k += rebuild_launches();
             } else {
                 launch_bvh_refit(d, st);
-                k += 2;
+                k += refit_launches();
             }
             launch_traverse(d, st); k += 2;
         } else {
@@ -791,6 +862,7 @@ struct Engine : EngineBase {
                 return cuda_status(e);
             }
         }
+        if (rebuild && d.nseg > 0) bvhBuilt = true;
         YB_CUDA(cudaGraphLaunch(graphs[type], S->stream));
         S->launches += graphLaunches[type];
         return YB_OK;
@@ -851,7 +923,12 @@ struct Engine : EngineBase {
     }
 
     void set_traversal(int packet) override {
-        if (d.travPacket != packet) invalidate_graphs();
+        if (d.travPacket == packet) return;
+        invalidate_graphs();
+        if ((d.travPacket == 2) != (packet == 2)) {  // the BVH is kept by the BVH walks only
+            bvhBuilt = false;
+            S->lastBVHRebuild = INFINITY;
+        }
         d.travPacket = packet;
     }
 
@@ -908,7 +985,7 @@ struct Engine : EngineBase {
             launch_bvh_rebuild(d, S->stream, sortScratch, sortBytes, keyBits);
             bvhBuilt = true;
         }
-        launch_scene_root_box(d, rootBoxes, S->stream);
+        launch_scene_box(d, rootBoxes, S->stream);
         S->launches++;
         std::vector<float> b(6 * (size_t)S->numScenes);
         YB_CUDA(cudaMemcpyAsync(b.data(), rootBoxes, sizeof(float) * b.size(), cudaMemcpyDeviceToHost, S->stream));
@@ -965,12 +1042,11 @@ struct Engine : EngineBase {
                 mark(1);
                 launch_bvh_rebuild(d, st, sortScratch, sortBytes, keyBits);
                 bvhBuilt = true;
-                const int passes = d.nseg > 1 ? (keyBits + 7) / 8 : 0;
-                launches[1] += 3 + (d.nseg > 1 ? 2 + passes : 0) + 1 + DEPTH_LAUNCHES + 2;
+                launches[1] += rebuild_launches();
             } else {
                 mark(2);
                 launch_bvh_refit(d, st);
-                launches[2] += 2;
+                launches[2] += refit_launches();
             }
             mark(3);
             launch_traverse(d, st); launches[3] += 2;
@@ -1053,10 +1129,10 @@ struct Engine : EngineBase {
             if ((mask & 2) || !bvhBuilt) {  // a refit needs a tree
                 launch_bvh_rebuild(d, st, sortScratch, sortBytes, keyBits);
                 bvhBuilt = true;
-                k += 3 + (d.nseg > 1 ? 2 + (keyBits + 7) / 8 : 0) + 1 + DEPTH_LAUNCHES + 2;
+                k += rebuild_launches();
             } else {
                 launch_bvh_refit(d, st);
-                k += 2;
+                k += refit_launches();
             }
             launch_traverse(d, st);
             k += 2;

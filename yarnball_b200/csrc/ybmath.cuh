@@ -279,15 +279,4 @@ template <typename R> YB_HD V3<R> qrotate(const Q<R>& q, V3<R> v) {
     return q.w * a + cross(qq, a) + c * qq;
 }
 
-// ---------------------------------------------------------------------------------------
-// 10-bit -> 30-bit Morton spread (bit i of v moves to bit 3i).
-YB_HD uint32_t morton_spread10(uint32_t v) {
-    v &= 0x3FFu;
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
 }  // namespace yb

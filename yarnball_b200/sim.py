@@ -387,8 +387,8 @@ class Sim:
         check(self._lib.yb_set_small_path(self._h, 1 if enable else 0), "small path")
 
     def set_traversal(self, mode=2):
-        """Broadphase walk: 2 (default) one per query with the warp's node records loaded
-        cooperatively, True / 1 one per warp of 32 queries (packet), False / 0 one per query."""
+        """Broadphase: 2 (default) pairs of clusters of 32 segments, True / 1 one BVH walk per warp
+        of 32 queries (packet), False / 0 one BVH walk per query."""
         m = (1 if mode else 0) if isinstance(mode, bool) else int(mode)
         check(self._lib.yb_set_traversal(self._h, m), "traversal")
 
