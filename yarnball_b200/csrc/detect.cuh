@@ -43,11 +43,26 @@ __device__ __forceinline__ Box<R> segment_box(const Dev<R>& d, int k, const Scen
     return b;
 }
 
-// Closed-interval overlap of a query box with a stored box.
+// The same box in single precision, rounded outwards (exact in the FP32 build); one that is not
+// a number meets nothing.  The w components are free.
+__device__ __forceinline__ float box_down(float x) { return x; }
+__device__ __forceinline__ float box_up(float x) { return x; }
+__device__ __forceinline__ float box_down(double x) { return __double2float_rd(x); }
+__device__ __forceinline__ float box_up(double x) { return __double2float_ru(x); }
+__device__ __forceinline__ float4 empty_lo() { return make_float4(INFINITY, INFINITY, INFINITY, 0.f); }
+__device__ __forceinline__ float4 empty_hi() { return make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f); }
+
+__device__ __forceinline__ bool boxes_meet(const float4& alo, const float4& ahi, const float4& blo, const float4& bhi) {
+    return alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z;
+}
 template <typename R>
-__device__ __forceinline__ bool box_overlap(const Box<R>& q, const R* mn, const R* mx) {
-    return q.mn[0] <= mx[0] && mn[0] <= q.mx[0] && q.mn[1] <= mx[1] && mn[1] <= q.mx[1] && q.mn[2] <= mx[2] &&
-           mn[2] <= q.mx[2];
+__device__ __forceinline__ void float_box(const Box<R>& b, float4& lo, float4& hi) {
+    lo = make_float4(box_down(b.mn[0]), box_down(b.mn[1]), box_down(b.mn[2]), 0.f);
+    hi = make_float4(box_up(b.mx[0]), box_up(b.mx[1]), box_up(b.mx[2]), 0.f);
+    if (!(lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z)) {
+        lo = empty_lo();
+        hi = empty_hi();
+    }
 }
 
 // Narrow-phase decision for segments x < y (both with hasNext, same scene): not joined by a

@@ -239,6 +239,7 @@ void launch_pin_drive(const Dev<R>& d, const float4* init, const unsigned char* 
 
 // One block advances a small simulation (n <= 256 vertices) through `steps` substeps in one launch.
 template <typename R> bool small_path_fits(const Dev<R>& d);
+template <typename R> cudaError_t small_path_prepare();  // once per device, before the first launch
 template <typename R>
 void launch_small(const Dev<R>& d, int steps, int numItr, unsigned long long step0, int detectionPeriod, bool kahan,
                   cudaStream_t s);

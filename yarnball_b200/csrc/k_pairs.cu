@@ -27,11 +27,6 @@
 
 namespace yb {
 
-__device__ __forceinline__ float box_down(float x) { return x; }
-__device__ __forceinline__ float box_up(float x) { return x; }
-__device__ __forceinline__ float box_down(double x) { return __double2float_rd(x); }
-__device__ __forceinline__ float box_up(double x) { return __double2float_ru(x); }
-
 // Order-preserving map of floats to unsigned, so that a warp's minimum is one redux.
 __device__ __forceinline__ unsigned box_ord(float f) {
     const unsigned u = __float_as_uint(f);
@@ -50,13 +45,6 @@ __device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
     lo.x = warp_min(lo.x); lo.y = warp_min(lo.y); lo.z = warp_min(lo.z);
     hi.x = warp_max(hi.x); hi.y = warp_max(hi.y); hi.z = warp_max(hi.z);
 }
-__device__ __forceinline__ float4 empty_lo() { return make_float4(INFINITY, INFINITY, INFINITY, 0.f); }
-__device__ __forceinline__ float4 empty_hi() { return make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f); }
-
-__device__ __forceinline__ bool boxes_meet(const float4& alo, const float4& ahi, const float4& blo, const float4& bhi) {
-    return alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z;
-}
-
 // One block per level-1 node (32 clusters, one per warp).  The block writes its clusters' boxes
 // and their union; the block that completes a level-2 (level-3) node, told by an arrival
 // counter that wraps to zero, writes that node's box from its 32 children.  Bound by the
@@ -80,12 +68,8 @@ __global__ void __launch_bounds__(BOX_THREADS) k_boxes(Dev<R> d, const int* __re
             k = sortedVals[sc.segBase + p];
             R reach;
             const Box<R> b = segment_box(d, k, d.sp[s], reach);
-            lo = make_float4(box_down(b.mn[0]), box_down(b.mn[1]), box_down(b.mn[2]), 0.f);
-            hi = make_float4(box_up(b.mx[0]), box_up(b.mx[1]), box_up(b.mx[2]), (float)reach);
-            if (!(lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z)) {  // not a number: meets nothing
-                lo = empty_lo();
-                hi = empty_hi();
-            }
+            float_box(b, lo, hi);
+            hi.w = (float)reach;
         }
         const size_t at = 32 * (size_t)(sc.lvl[0] + c) + lane;
         lo.w = __int_as_float(k);

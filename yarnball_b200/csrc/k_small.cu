@@ -2,16 +2,27 @@
 // advance() in a single launch.
 //
 // A scene of a few hundred vertices keeps a B200 busy for microseconds per kernel, so the
-// per-substep kernel sequence (predictor, BVH refit and traversal, list pass, numItr Newton
-// launches, advection) is bound by launch latency: the README two-yarn scene (64 vertices)
-// takes ~64 us per substep that way.  Here one block of SMALL_THREADS threads, one vertex per
-// thread, runs all substeps with block barriers between the phases: the same device functions
-// as the multi-block kernels (step.cuh, detect.cuh) in the same order and with the
-// load-balanced Newton kernel's summation order, and the same contact set (every pair of
-// segments goes through the narrow-phase filter; a pair the filter keeps has overlapping padded
-// boxes, which is all the BVH query contributes).  The compiler may contract multiplies and
-// adds into fused operations differently in this one kernel than in the separate kernels, so
-// the two paths agree to rounding rather than bit for bit.
+// per-substep kernel sequence is bound by launch latency.  Here one block runs all substeps,
+// with the whole state, the contact lists and the staged partner positions in shared memory:
+// global memory is read at the start and written at the end.  The device functions are the
+// multi-block kernels' (step.cuh, detect.cuh), given a copy of the engine's pointers that
+// points into shared memory.
+//
+// The block is bound by the latency of its dependent chain, not by issue, so the chain is
+// shortened and split over roles:
+//   * `vt` vertex threads (one vertex each) and CT contact threads.  In a Newton iteration the
+//     contact threads evaluate the contacts, CT at a time and one per thread, while the vertex
+//     threads evaluate inertia, glue and stretch, then sum the contributions in list order; the
+//     next iteration's contacts start as soon as the new displacements are known, beside the
+//     orientation update;
+//   * the pair search tests all padded boxes, every pair of vertices once, spread over all
+//     threads; hits go through a queue per warp so that the exact narrow phase runs on 32 pairs
+//     at once;
+//   * contact lists are rows of a bit matrix: a kept pair sets two bits, and reading a row
+//     upwards gives the list in partner order without a sort.
+// Measured (B200, us per substep, before -> now, where before one thread ran each vertex with
+// all of its pairs and contacts in global memory): README scene (64 vertices, few contacts)
+// 53 -> 16; swatch of 216 vertices (2 contacts a segment) 209 -> 46.
 //
 // Reference semantics: Sim::advance (sim/step.cpp:36-55) with initItr / endItr
 // (sim/iteration.cu), detectCollisions + buildCollisionList (sim/collision.cu:39-119),
@@ -21,210 +32,370 @@
 
 namespace yb {
 
-constexpr int SMALL_THREADS = 256;  // largest simulation this path runs (vertices)
+constexpr int SMALL_VERTS = 256;  // largest simulation this path runs (vertices)
+constexpr int SMALL_WORDS = SMALL_VERTS / 32;
+constexpr int SMALL_SCENES = 16;  // scene parameters kept in shared memory up to this many
 
 template <typename R>
-__device__ __forceinline__ void small_append(const Dev<R>& d, int x, int y) {
-    const int at = atomicAdd(&d.numCols[x], 1);
-    if (at < MAX_COLS) d.cols[col_at(x, at)] = y;
+struct SmallShare {
+    static constexpr int CT = sizeof(R) == 4 ? 256 : 128;   // contact threads
+    static constexpr int CAP = sizeof(R) == 4 ? 2560 : 640; // contacts held here; the rest is read from global memory
+    static constexpr int WARPS = (SMALL_VERTS + CT) / 32;
+    V4<R> pos[SMALL_VERTS], posC[SMALL_VERTS], vel[SMALL_VERTS], lastVel[SMALL_VERTS];
+    V4<R> q[2][SMALL_VERTS], qRest[SMALL_VERTS];
+    D2<R> dx[2][SMALL_VERTS];
+    VP<R> vp[SMALL_VERTS];
+    R stepLim[SMALL_VERTS];
+    V4<R> con4[2][4][CT];  // contributions of a chunk of contacts, as k_iter_bal groups them
+    R2<R> con2[2][CT];
+    V4<R> relA[CAP];
+    R2<R> relB[CAP];
+    int pack[CAP];         // owner << 16 | partner
+    R halo[10][SMALL_VERTS];  // fb, Hb and the step limit of each segment
+    R newDx[3][SMALL_VERTS];
+    float4 boxLo[SMALL_VERTS], boxHi[SMALL_VERTS];
+    unsigned adj[SMALL_VERTS][SMALL_WORDS];
+    int queue[WARPS][64];
+    int warpSum[SMALL_WORDS];
+    SceneParams<R> sp[SMALL_SCENES];
+};
+
+__device__ __forceinline__ void small_min(float* at, float v) {
+    atomicMin(reinterpret_cast<unsigned*>(at), __float_as_uint(v));
+}
+__device__ __forceinline__ void small_min(double* at, double v) {
+    atomicMin(reinterpret_cast<unsigned long long*>(at), (unsigned long long)__double_as_longlong(v));
 }
 
 template <typename R>
-__global__ void __launch_bounds__(SMALL_THREADS) k_small(Dev<R> d, int steps, int numItr, unsigned long long step0,
-                                                         int detectionPeriod, int kahan) {
-    __shared__ R sFb[3][SMALL_THREADS];
-    __shared__ R sHb[6][SMALL_THREADS];
-    __shared__ R sSL[SMALL_THREADS];
-    __shared__ R sDX[3][SMALL_THREADS];
-    typedef Ex<R> E;
-    const int k = threadIdx.x;
-    const int n = d.n;
-    const bool valid = k < n;
-    const uint32_t fl0 = valid ? d.vp[k].flags : 0u;
+__global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
+    k_small(const __grid_constant__ Dev<R> g, int steps, int numItr, unsigned long long step0, int detectionPeriod,
+            int kahan) {
+    constexpr int CT = SmallShare<R>::CT, CAP = SmallShare<R>::CAP;
+    const unsigned FULL = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char raw[];
+    SmallShare<R>& m = *reinterpret_cast<SmallShare<R>*>(raw);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int n = g.n;
+    const int vt = (int)blockDim.x - CT;  // vertex threads: n rounded up to whole warps
+    const int k = t;
+    const bool vertexWarp = t < vt, valid = t < n;
+    Dev<R> d = g;
+    d.pos = m.pos; d.posC = m.posC; d.vel = m.vel; d.lastVel = m.lastVel;
+    d.dx[0] = m.dx[0]; d.dx[1] = m.dx[1];
+    d.q[0] = m.q[0]; d.q[1] = m.q[1];
+    d.qRest = m.qRest; d.vp = m.vp; d.stepLim = m.stepLim;
+    d.relA = m.relA; d.relB = m.relB; d.relCap = CAP;
+    if (g.numScenes <= SMALL_SCENES) {
+        for (int s = t; s < g.numScenes; s += blockDim.x) m.sp[s] = g.sp[s];
+        d.sp = m.sp;
+    }
+    uint32_t fl0 = 0;
+    int nc = 0;
+    if (valid) {
+        m.pos[k] = g.pos[k]; m.posC[k] = g.posC[k]; m.vel[k] = g.vel[k]; m.lastVel[k] = g.lastVel[k];
+        m.q[0][k] = g.q[0][k]; m.q[1][k] = g.q[0][k]; m.qRest[k] = g.qRest[k];
+        m.dx[0][k] = g.dx[0][k]; m.dx[1][k] = g.dx[1][k];
+        const VP<R> vp = g.vp[k];
+        m.vp[k] = vp;
+        fl0 = vp.flags;
+        // the lists of the last detection, in case the first substep does not detect
+        nc = min(max(g.numCols[k], 0), MAX_COLS);
+    }
+    if (vertexWarp) {
+        m.stepLim[k] = yinf<R>();
+#pragma unroll
+        for (int w = 0; w < SMALL_WORDS; w++) m.adj[k][w] = 0u;
+        for (int c = 0; c < nc; c++) {
+            const int j = g.cols[col_at(k, c)];
+            if ((unsigned)j < (unsigned)n) m.adj[k][j >> 5] |= 1u << (j & 31);
+        }
+    }
     const bool seg = valid && (fl0 & F_HAS_NEXT);
     const int sc = scene_of(fl0);
+    __syncthreads();
+
+    int off = 0, total = 0;  // this segment's first packed contact; all contacts
+    int pens = 0, most = 0;
+    float dmin = INFINITY;
+    bool lists = false;      // the packed contacts follow the bit matrix
     for (int s = 0; s < steps; s++) {
-        // predictor (k_init)
         if (valid) init_vertex(d, k);
         __syncthreads();
         const bool detect = detectionPeriod > 0 && (step0 + (unsigned long long)s) % (unsigned long long)detectionPeriod == 0;
         if (detect) {
-            if (valid) d.numCols[k] = 0;
-            __syncthreads();
-            // narrow phase over every pair of segments of the scene, lower index first (k_traverse)
-            if (seg) {
-                const SceneParams<R>& sp = d.sp[sc];
-                for (int y = k + 3; y < n; y++) {
-                    const uint32_t fy = d.vp[y].flags;
-                    if (!(fy & F_HAS_NEXT) || scene_of(fy) != sc) continue;
-                    if (pair_keep(d, k, y, sp)) {
-                        small_append(d, k, y);
-                        small_append(d, y, k);
-                    }
+            if (vertexWarp) {
+                float4 lo = empty_lo(), hi = empty_hi();
+                if (seg) {
+                    R reach;
+                    float_box(segment_box(d, k, d.sp[sc], reach), lo, hi);
+                    lo.w = __int_as_float(sc);
                 }
+                m.boxLo[k] = lo;
+                m.boxHi[k] = hi;
+#pragma unroll
+                for (int w = 0; w < SMALL_WORDS; w++) m.adj[k][w] = 0u;
             }
             __syncthreads();
-            // list clamp, overflow error and sort by partner id (k_lists)
-            if (seg) {
-                int nc = d.numCols[k];
-                if (nc) atomicMax(&d.err[EW_MAX_COLS], nc);
-                if (nc > MAX_COLS) d.err[EW_ERROR] = 1;
-                nc = min(nc, MAX_COLS);
-                d.numCols[k] = nc;
-                int* row = d.cols + col_at(k, 0);
-                for (int i = 1; i < nc; i++) {
-                    const int v = row[i];
-                    int j = i - 1;
-                    while (j >= 0 && row[j] > v) {
-                        row[j + 1] = row[j];
-                        j--;
+            // vertex x against x + o (cyclic), o = 1 .. n / 2: every pair of vertices once
+            int qn = 0;
+            int* queue = m.queue[warp];
+            auto drain = [&](int first, int count) {
+                if (lane < count) {
+                    const int e = queue[first + lane];
+                    const int x = e >> 16, y = e & 0xffff;
+                    if (pair_keep(d, x, y, d.sp[scene_of(m.vp[x].flags)])) {
+                        atomicOr(&m.adj[x][y >> 5], 1u << (y & 31));
+                        atomicOr(&m.adj[y][x >> 5], 1u << (x & 31));
                     }
-                    row[j + 1] = v;
                 }
+                __syncwarp();
+            };
+            const int parts = (int)blockDim.x / vt, part = t / vt;
+            if (part < parts) {  // whole warps
+                const int x = t - part * vt;
+                const float4 lo = x < n ? m.boxLo[x] : empty_lo(), hi = x < n ? m.boxHi[x] : empty_hi();
+                const int half = n / 2;
+                // 32 partners at a time into a mask, then one hit of each thread at a time
+                for (int o0 = 1 + part; o0 <= half; o0 += 32 * parts) {
+                    unsigned hits = 0;
+                    const int count = min(32, (half - o0) / parts + 1);
+#pragma unroll 4
+                    for (int i = 0; i < count; i++) {
+                        int y = x + o0 + i * parts;
+                        if (y >= n) y -= n;
+                        y = min(y, SMALL_VERTS - 1);  // threads past the last vertex read, and meet nothing
+                        if (boxes_meet(lo, hi, m.boxLo[y], m.boxHi[y])) hits |= 1u << i;
+                    }
+                    // with n even, x and x + n / 2 meet from both sides
+                    if (2 * (o0 + (count - 1) * parts) == n && x >= half) hits &= ~(1u << (count - 1));
+                    while (__any_sync(FULL, hits != 0)) {
+                        int y = x + o0 + (__ffs(hits) - 1) * parts;
+                        if (y >= n) y -= n;
+                        const int a = min(x, y), b = max(x, y);
+                        const bool take = hits && b - a > 2 && __float_as_int(lo.w) == __float_as_int(m.boxLo[y].w);
+                        hits &= hits - 1;
+                        const unsigned mask = __ballot_sync(FULL, take);
+                        if (take) queue[qn + __popc(mask & lt)] = a << 16 | b;
+                        qn += __popc(mask);
+                        __syncwarp();
+                        if (qn >= 32) {
+                            qn -= 32;
+                            drain(qn, 32);
+                        }
+                    }
+                }
+                if (qn) drain(0, qn);
             }
+            __syncthreads();
+            lists = false;
         }
-        // step limit, staged partner positions, interpenetration statistics (k_lists)
-        if (seg) {
-            const SceneParams<R>& sp = d.sp[sc];
-            const int nc = d.numCols[k];
-            const V3<R> a0 = xyz(d.pos[k]);
-            const V3<R> a1 = xsub(xyz(d.pos[k + 1]), a0);
-            R m = step_limit_base(d, k, sp);
-            int pens = 0;
-            float dmin = INFINITY;
-            for (int c = 0; c < nc; c++) {
-                const int o = d.cols[col_at(k, c)];
-                bool pen;
-                R dist;
-                const R lim =
-                    contact_step_limit(d, k, c < RELCAP ? rel_at(k, c) : NO_STAGE, o, a0, a1, sp, pen, dist);
-                pens += pen;
-                dmin = fminf(dmin, (float)dist);
-                m = ymin(m, lim);
+        if (!lists) {
+            // list lengths, their clamp (the lowest partner ids stay) and the packed contacts
+            if (vertexWarp) {
+                int c = 0;
+#pragma unroll
+                for (int w = 0; w < SMALL_WORDS; w++) c += __popc(m.adj[k][w]);
+                if (detect) {
+                    most = max(most, c);
+                    if (c > MAX_COLS) g.err[EW_ERROR] = 1;
+                }
+                nc = min(c, MAX_COLS);
+                off = nc;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(FULL, off, o);
+                    if (lane >= o) off += y;
+                }
+                if (lane == 31) m.warpSum[warp] = off;
+                off -= nc;
             }
-            if (pens) {
-                atomicAdd(&d.err[EW_PENETRATIONS], pens);
-                d.err[EW_WARNING] = 2;
+            __syncthreads();
+            total = 0;
+            for (int w = 0; w < vt / 32; w++) {
+                if (w < warp && vertexWarp) off += m.warpSum[w];
+                total += m.warpSum[w];
             }
-            if (dmin < INFINITY) atomicMin(&d.err[EW_MIN_DIST], __float_as_int(dmin));
-            d.stepLim[k] = sp.useStepLimit ? m : yinf<R>();
+            if (vertexWarp && nc) {
+                int at = off;
+                const int end = off + nc;
+                for (int w = 0; w < SMALL_WORDS; w++)
+                    for (unsigned bits = m.adj[k][w]; bits && at < end; bits &= bits - 1, at++) {
+                        const int e = k << 16 | (32 * w + __ffs(bits) - 1);
+                        if (at < CAP) m.pack[at] = e; else g.csrCols[at] = e;
+                    }
+            }
+            lists = true;
+        }
+        if (seg) m.stepLim[k] = step_limit_base(d, k, d.sp[sc]);
+        __syncthreads();
+        // step limit, staged partner positions, interpenetration statistics
+        for (int f = t; f < total; f += blockDim.x) {
+            const int e = f < CAP ? m.pack[f] : g.csrCols[f];
+            const int a = e >> 16, o = e & 0xffff;
+            const V3<R> a0 = xyz(m.pos[a]);
+            const V3<R> a1 = xsub(xyz(m.pos[a + 1]), a0);
+            bool pen;
+            R dist;
+            const R lim = contact_step_limit(d, a, f < CAP ? (size_t)f : NO_STAGE, o, a0, a1,
+                                             d.sp[scene_of(m.vp[a].flags)], pen, dist);
+            pens += pen;
+            dmin = fminf(dmin, (float)dist);
+            small_min(&m.stepLim[a], lim);  // limits are >= 0: their bits order like them
         }
         __syncthreads();
-        // Newton + orientation iterations (k_iter_bal's arithmetic and summation order)
+        if (valid && !(seg && d.sp[sc].useStepLimit)) m.stepLim[k] = yinf<R>();
+
+        const int chunks = (total + CT - 1) / CT;
+        int buf = 0;
         for (int it = 0; it < numItr; it++) {
             const int src = it & 1;
-            const D2<R>* __restrict__ DX = d.dx[src];
-            const V4<R>* __restrict__ QO = d.q[src];
-            V3<R> p0(R(0)), e(R(0)), dx(R(0)), dx1(R(0));
-            int nc = 0;
-            if (valid) {
-                const D2<R> own = DX[k];
-                dx = xyz(own.a);
-                dx1 = xyz(own.b);
-                p0 = xyz(d.pos[k]);
-                if (seg) {
-                    e = xyz(d.pos[k + 1]) - p0;
-                    nc = d.numCols[k];
-                }
-            }
+            const D2<R>* DX = m.dx[src];
+            const V4<R>* QO = m.q[src];
+            auto evaluate = [&](int chunk, int to) {
+                const int u = t - vt, f = chunk * CT + u;
+                if (u < 0 || f >= total) return;
+                const int e = f < CAP ? m.pack[f] : g.csrCols[f];
+                const int a = e >> 16, o = e & 0xffff;
+                const V3<R> p0 = xyz(m.pos[a]);
+                V3<R> r0, r1;
+                partner_rel(d, (unsigned)f, o, p0, r0, r1);
+                const D2<R> own = DX[a], pd = DX[o];
+                V3<R> fa(R(0)), fb(R(0));
+                H3<R> Ha, Hb;
+                Ha.zero();
+                Hb.zero();
+                contact_term(xyz(m.pos[a + 1]) - p0, xyz(own.a), xyz(own.b), r0, r1, xyz(pd.a), xyz(pd.b),
+                             d.sp[scene_of(m.vp[a].flags)], fa, Ha, fb, Hb);
+                V4<R> w;
+                w.x = fa.x; w.y = fa.y; w.z = fa.z; w.w = fb.x; m.con4[to][0][u] = w;
+                w.x = fb.y; w.y = fb.z; w.z = Ha.d[0]; w.w = Ha.d[1]; m.con4[to][1][u] = w;
+                w.x = Ha.d[2]; w.y = Ha.d[3]; w.z = Ha.d[4]; w.w = Ha.d[5]; m.con4[to][2][u] = w;
+                w.x = Hb.d[0]; w.y = Hb.d[1]; w.z = Hb.d[2]; w.w = Hb.d[3]; m.con4[to][3][u] = w;
+                R2<R> w2;
+                w2.x = Hb.d[4]; w2.y = Hb.d[5];
+                m.con2[to][u] = w2;
+            };
             V3<R> fa(R(0)), fb(R(0));
             H3<R> Ha, Hb;
             Ha.zero();
             Hb.zero();
-            if (nc) {
-                const SceneParams<R>& sp = d.sp[sc];
-                for (int c = 0; c < nc; c++) {
-                    const int j = d.cols[col_at(k, c)];
-                    V3<R> r0, r1;
-                    if (c < RELCAP) {
-                        const size_t at = rel_at(k, c);
-                        const V4<R> A = d.relA[at];
-                        const R2<R> Bq = d.relB[at];
-                        r0 = V3<R>(A.x, A.y, A.z);
-                        r1 = V3<R>(A.w, Bq.x, Bq.y);
-                    } else {
-                        r0 = xyz(d.pos[j]) - p0;
-                        r1 = xyz(d.pos[j + 1]) - p0;
-                    }
-                    const D2<R> pd = DX[j];
-                    V3<R> cfa(R(0)), cfb(R(0));
-                    H3<R> cHa, cHb;
-                    cHa.zero();
-                    cHb.zero();
-                    contact_term(e, dx, dx1, r0, r1, xyz(pd.a), xyz(pd.b), sp, cfa, cHa, cfb, cHb);
-                    // Separately rounded sums: k_iter_bal adds each contribution after a trip
-                    // through shared memory, so the compiler cannot fuse the contribution's last
-                    // multiply into the sum there; it must not here either.
-                    fa = V3<R>(E::add(fa.x, cfa.x), E::add(fa.y, cfa.y), E::add(fa.z, cfa.z));
-                    fb = V3<R>(E::add(fb.x, cfb.x), E::add(fb.y, cfb.y), E::add(fb.z, cfb.z));
-#pragma unroll
-                    for (int q = 0; q < 6; q++) {
-                        Ha.d[q] = E::add(Ha.d[q], cHa.d[q]);
-                        Hb.d[q] = E::add(Hb.d[q], cHb.d[q]);
-                    }
-                }
-            }
             R sl = yinf<R>();
             uint32_t flags = 0;
             R invMass = R(0), lRest = R(1), kStretch = R(0);
             Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
-            if (valid)
-                add_own_terms(d, k, DX, QO, d.sp[sc], p0, e, dx, dx1, fa, Ha, fb, Hb, flags, invMass, lRest, kStretch,
-                              sl, q0);
-            sFb[0][k] = fb.x; sFb[1][k] = fb.y; sFb[2][k] = fb.z;
-#pragma unroll
-            for (int q = 0; q < 6; q++) sHb[q][k] = Hb.d[q];
-            sSL[k] = sl;
-            __syncthreads();
+            V3<R> p0(R(0)), e(R(0)), dx(R(0));
+            if (chunks) evaluate(0, buf);
+            if (valid) {
+                const D2<R> own = DX[k];
+                dx = xyz(own.a);
+                p0 = xyz(m.pos[k]);
+                if (seg) e = xyz(m.pos[k + 1]) - p0;
+                add_own_terms(d, k, DX, QO, d.sp[sc], p0, e, dx, xyz(own.b), fa, Ha, fb, Hb, flags, invMass, lRest,
+                              kStretch, sl, q0);
+            }
+            for (int c = 0; c < chunks; c++, buf ^= 1) {
+                __syncthreads();  // chunk c is evaluated, and chunk c - 1 summed
+                if (c + 1 < chunks) evaluate(c + 1, buf ^ 1);
+                if (vertexWarp) {
+                    const int f1 = min(off + nc, (c + 1) * CT) - c * CT;
+                    for (int i = max(off - c * CT, 0); i < f1; i++) {
+                        const V4<R> w0 = m.con4[buf][0][i], w1 = m.con4[buf][1][i], w2 = m.con4[buf][2][i],
+                                    w3 = m.con4[buf][3][i];
+                        const R2<R> w4 = m.con2[buf][i];
+                        fa += V3<R>(w0.x, w0.y, w0.z);
+                        fb += V3<R>(w0.w, w1.x, w1.y);
+                        Ha.d[0] += w1.z; Ha.d[1] += w1.w;
+                        Ha.d[2] += w2.x; Ha.d[3] += w2.y; Ha.d[4] += w2.z; Ha.d[5] += w2.w;
+                        Hb.d[0] += w3.x; Hb.d[1] += w3.y; Hb.d[2] += w3.z; Hb.d[3] += w3.w;
+                        Hb.d[4] += w4.x; Hb.d[5] += w4.y;
+                    }
+                }
+            }
             V3<R> dxn = dx;
-            if (valid) {
-                if (flags & F_HAS_PREV) {
-                    fa += V3<R>(sFb[0][k - 1], sFb[1][k - 1], sFb[2][k - 1]);
-                    H3<R> hp;
+            if (vertexWarp) {
+                m.halo[0][k] = fb.x; m.halo[1][k] = fb.y; m.halo[2][k] = fb.z;
 #pragma unroll
-                    for (int q = 0; q < 6; q++) hp.d[q] = sHb[q][k - 1];
-                    Ha.add(hp);
-                    sl = ymin(sl, sSL[k - 1]);
-                }
-                if (invMass != R(0)) {
-                    dxn = dx + d.sp[sc].accel * solve3(Ha, fa);
-                    const R l = len(dxn);
-                    if (l > sl && l > R(0)) dxn *= sl / l;
+                for (int q = 0; q < 6; q++) m.halo[3 + q][k] = Hb.d[q];
+                m.halo[9][k] = sl;
+                asm volatile("bar.sync 1, %0;" ::"r"(vt) : "memory");  // the vertex threads only
+                if (valid) {
+                    if (flags & F_HAS_PREV) {
+                        fa += V3<R>(m.halo[0][k - 1], m.halo[1][k - 1], m.halo[2][k - 1]);
+                        H3<R> hp;
+#pragma unroll
+                        for (int q = 0; q < 6; q++) hp.d[q] = m.halo[3 + q][k - 1];
+                        Ha.add(hp);
+                        sl = ymin(sl, m.halo[9][k - 1]);
+                    }
+                    if (invMass != R(0)) {
+                        dxn = dx + d.sp[sc].accel * solve3(Ha, fa);
+                        const R l = len(dxn);
+                        if (l > sl && l > R(0)) dxn *= sl / l;
+                    }
+                    // the new iterate pair: this vertex's half of its own and of the one before
+                    m.dx[src ^ 1][k].a = v4(dxn, R(0));
+                    if (k > 0) m.dx[src ^ 1][k - 1].b = v4(dxn, R(0));
+                    if (k == n - 1) m.dx[src ^ 1][k].b = v4(V3<R>(R(0)), R(0));
                 }
             }
-            sDX[0][k] = dxn.x; sDX[1][k] = dxn.y; sDX[2][k] = dxn.z;
             __syncthreads();
-            if (valid) {
-                const V3<R> dxb = k + 1 < n ? V3<R>(sDX[0][k + 1], sDX[1][k + 1], sDX[2][k + 1]) : V3<R>(R(0));
-                D2<R> o;
-                o.a = v4(dxn, R(0));
-                o.b = v4(dxb, R(0));
-                d.dx[src ^ 1][k] = o;
-                d.q[src ^ 1][k] = v4of(orientation_update(d, k, QO, flags, e, dxn, dxb, lRest, kStretch, q0));
-            }
-            __syncthreads();
+            if (valid)
+                m.q[src ^ 1][k] = v4of(orientation_update(d, k, QO, flags, e, dxn, xyz(m.dx[src ^ 1][k].b), lRest,
+                                                          kStretch, q0));
         }
-        // advection (k_end)
-        if (valid) end_vertex(d, k, numItr & 1, (numItr & 1) != 0, kahan);
+        if (numItr & 1) {
+            __syncthreads();  // neighbours still read q[0], which end_vertex overwrites
+            if (valid) end_vertex(d, k, 1, 1, kahan);
+        } else if (valid) {
+            end_vertex(d, k, 0, 0, kahan);
+        }
         __syncthreads();
     }
+
+    if (valid) {
+        g.pos[k] = m.pos[k]; g.posC[k] = m.posC[k]; g.vel[k] = m.vel[k]; g.lastVel[k] = m.lastVel[k];
+        g.q[0][k] = m.q[0][k]; g.dx[0][k] = m.dx[0][k]; g.dx[1][k] = m.dx[1][k];
+        g.stepLim[k] = m.stepLim[k];
+        g.numCols[k] = nc;
+        int c = 0;
+        for (int w = 0; w < SMALL_WORDS; w++)
+            for (unsigned bits = m.adj[k][w]; bits && c < nc; bits &= bits - 1)
+                g.cols[col_at(k, c++)] = 32 * w + __ffs(bits) - 1;
+    }
+    if (most) atomicMax(&g.err[EW_MAX_COLS], most);
+    if (pens) {
+        atomicAdd(&g.err[EW_PENETRATIONS], pens);
+        g.err[EW_WARNING] = 2;
+    }
+    if (dmin < INFINITY) atomicMin(&g.err[EW_MIN_DIST], __float_as_int(dmin));
 }
 
 template <typename R>
 bool small_path_fits(const Dev<R>& d) {
-    return d.n > 0 && d.n <= SMALL_THREADS;
+    return d.n > 0 && d.n <= SMALL_VERTS;
+}
+
+template <typename R>
+cudaError_t small_path_prepare() {
+    static_assert(sizeof(SmallShare<R>) <= 227 * 1024, "shared memory of one block");
+    return cudaFuncSetAttribute(k_small<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallShare<R>));
 }
 
 template <typename R>
 void launch_small(const Dev<R>& d, int steps, int numItr, unsigned long long step0, int detectionPeriod, bool kahan,
                   cudaStream_t s) {
     if (d.n <= 0 || steps <= 0) return;
-    k_small<R><<<1, SMALL_THREADS, 0, s>>>(d, steps, numItr, step0, detectionPeriod, kahan ? 1 : 0);
+    const int threads = (d.n + 31) / 32 * 32 + SmallShare<R>::CT;
+    k_small<R><<<1, threads, sizeof(SmallShare<R>), s>>>(d, steps, numItr, step0, detectionPeriod, kahan ? 1 : 0);
 }
 
-template bool small_path_fits<float>(const Dev<float>&);
-template bool small_path_fits<double>(const Dev<double>&);
-template void launch_small<float>(const Dev<float>&, int, int, unsigned long long, int, bool, cudaStream_t);
-template void launch_small<double>(const Dev<double>&, int, int, unsigned long long, int, bool, cudaStream_t);
+#define YB_INST(R)                                                                                            \
+    template bool small_path_fits<R>(const Dev<R>&);                                                          \
+    template cudaError_t small_path_prepare<R>();                                                             \
+    template void launch_small<R>(const Dev<R>&, int, int, unsigned long long, int, bool, cudaStream_t);
+YB_INST(float)
+YB_INST(double)
 
 }  // namespace yb

@@ -421,6 +421,7 @@ struct Engine : EngineBase {
             d.pairWarps = sms * 32;
         }
         d.travPacket = S->travPacket;
+        YB_CUDA(small_path_prepare<R>());  // a recycled batch may become small later
         YB_CUDA(cudaHostAlloc((void**)&spHost, sizeof(SceneParams<R>) * ns, cudaHostAllocDefault));
         YB_CUDA(cudaHostAlloc((void**)&errHost, sizeof(int) * EW_COUNT, cudaHostAllocDefault));
         YB_CUDA(cudaMemsetAsync(d.err, 0, sizeof(int) * EW_COUNT, S->stream));
