@@ -151,6 +151,10 @@ __device__ __forceinline__ R contact_step_limit(const Dev<R>& d, int k, size_t s
     const UVT<R> uv = closest_uv_exact(a1, b0, b1);
     const V3<R> nrm = xsub(xscale(uv.u, a1), xmix(b0, b1, uv.v));
     const R l = E::sqrt(xlen2(nrm));
+    if (stage != NO_STAGE && d.relD) {
+        const R room = l - sp.outOfRange;
+        d.relD[stage] = room > R(0) ? room * room : R(-1);
+    }
     pen = o > k && l <= sp.twoR;
     dist = l;
     const R safe = E::mul(E::sub(R(1), R(0.1f)), R(0.5f));

@@ -17,8 +17,9 @@
 //   csrOff   u32    n + 1: the contacts of vertex k, packed in vertex order by the list pass
 //                   every substep, are slots [csrOff[k], csrOff[k+1]) of
 //   csrCols  int    partner ids (sorted within each vertex's range)
-//   relA/B   V4,R2  partner endpoints relative to p0, staged per substep in the same slots
-//                   while the slot is below relCap (the one-block path stages rows of RELCAP)
+//   csrOwner u8     low byte of the vertex each packed contact belongs to
+//   relA/B/D V4,R2,R  partner endpoints relative to p0 and the squared room to the barrier's reach,
+//                   staged per substep in the same slots while the slot is below relCap
 // Segments are the vertices with hasNext; segs[] lists them, scene after scene.
 #pragma once
 #include "ybmath.cuh"
@@ -63,7 +64,7 @@ struct alignas(sizeof(R) * 2) R2 {
     R x, y;
 };
 
-constexpr int RELCAP = 8;  // staged relative partner positions: RELCAP x vertices slots in all
+constexpr int RELCAP = 16;  // staged contacts: RELCAP x vertices slots in all (a contact past them is gathered)
 constexpr int LIST_THREADS = 128;  // vertices per block of the list pass (one packed-offset tile)
 
 // Wide records are built only for the nodes the walk loads: those at an even depth below
@@ -73,11 +74,8 @@ constexpr int LIST_THREADS = 128;  // vertices per block of the list pass (one p
 constexpr int DEPTH_ROUNDS = 7;
 constexpr int DEPTH_LAUNCHES = 1 + DEPTH_ROUNDS + 1;  // init, jumps, marks
 
-// Contact-list addressing: each segment owns a row of MAX_COLS partner ids and a row of RELCAP
-// staged partner positions, so the contacts of one segment are contiguous (the flattened
-// contact loop of the Newton kernel reads consecutive contacts of one owner together).
+// Contact-list addressing: each segment owns a row of MAX_COLS partner ids.
 __host__ __device__ __forceinline__ size_t col_at(int seg, int c) { return (size_t)seg * MAX_COLS + c; }
-__host__ __device__ __forceinline__ size_t rel_at(int seg, int c) { return (size_t)seg * RELCAP + c; }
 
 template <typename R>
 struct VP {
@@ -94,6 +92,7 @@ struct SceneParams {
     R D;                            // damping / h
     R accel;                        // accelerationRatio
     R twoR;                         // 2 * radius
+    R outOfRange;                   // a contact farther apart than this has a gap above 1, with a margin for rounding
     R invb;                         // 1 / barrierThickness
     R kCol;                         // kCollision / barrierThickness
     R fricK, fricMu;                // kFriction, frictionCoeff
@@ -158,6 +157,7 @@ template <typename R>
 struct Dev {
     int n;            // vertices
     int nseg;         // segments (= BVH leaves)
+    int sms;          // multiprocessors of the device
     int numScenes;
     V4<R>* pos;
     V4<R>* posC;
@@ -172,8 +172,11 @@ struct Dev {
     int* cols;
     V4<R>* relA;      // staged per substep in the packed slots below relCap:
     R2<R>* relB;      //   relA = (b0 - p0, (b1 - p0).x), relB = (b1 - p0).yz
+    R* relD;          //   squared room: how far the centre lines are beyond the barrier's reach at the
+                      //   start of the substep, -1 when they are not (null: not kept)
     unsigned* csrOff; // n + 1 packed offsets (see the layout above)
     int* csrCols;     // csrCap packed partner ids
+    unsigned char* csrOwner;  // low byte of each packed contact's vertex
     unsigned csrCap;  // slots of csrCols
     unsigned relCap;  // slots of relA / relB
     unsigned long long* listStatus;  // list pass: [0] tile ticket, [1 + tile] look-back status
@@ -199,7 +202,6 @@ struct Dev {
                           // queries (k_traverse_packet), 0: one per lane (k_traverse)
     // clusters of 32 segments in curve order (k_pairs.cu)
     int nclus, nl1;       // clusters and level-1 nodes of all scenes
-    int pairWarps;        // fewest warps the pair search is spread over
     float4 *leafLo, *leafHi;  // 32 per cluster: padded box of each segment; leafLo.w = its vertex
                               // (-1: none), leafHi.w = its reach (segment_box)
     int* sceneGlued;      // 1: some vertex of the scene has a connection

@@ -758,7 +758,10 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
             const int ks = tile * B + s;
             const int o = d.cols[col_at(ks, c)];
             const unsigned long long g = base + (unsigned long long)f;
-            if (g < (unsigned long long)d.csrCap) d.csrCols[g] = o;
+            if (g < (unsigned long long)d.csrCap) {
+                d.csrCols[g] = o;
+                d.csrOwner[g] = (unsigned char)ks;
+            }
             const V3<R> oa0(sA0[0][s], sA0[1][s], sA0[2][s]);
             const V3<R> oa1(sA1[0][s], sA1[1][s], sA1[2][s]);
             bool pen = false;

@@ -126,8 +126,10 @@ __global__ void __launch_bounds__(BOX_THREADS) k_boxes(Dev<R> d, const int* __re
 // 16-byte reads and six compares a test), collecting the hits in a bit mask.  Hits go through a
 // queue of the warp, so that the separately rounded narrow-phase test runs on 32 pairs at once.
 // Bound by issue and latency (ncu, a million vertices: half of the issue slots busy at 38 % of
-// the warps).  `parts` doubles until there are 32 warps for every SM: with 4 or 16 times as many
-// the piles take 0-20 % and 40-50 % longer (every part repeats the walk).
+// the warps).  `parts` makes 96 warps for every SM, three times what an SM holds, since the
+// clusters' work is uneven: the class of this kernel and the list pass takes 330 / 232 / 222 us
+// with 32 / 96 / 192 warps per SM on a bundle of 100,352 vertices, 144 / 146 / 163 us on a pile
+// of 65,792 and 365 / 342 / 361 us on one of 262,144 (every part repeats the walk).
 constexpr int PAIR_THREADS = 128;
 constexpr int PAIR_WARPS = PAIR_THREADS / 32;
 
@@ -321,8 +323,7 @@ void launch_boxes(const Dev<R>& d, cudaStream_t s) {
 template <typename R>
 void launch_pairs(const Dev<R>& d, cudaStream_t s) {
     if (d.nclus <= 0) return;
-    int parts = 1;
-    while (parts < 32 && (long long)d.nclus * parts < d.pairWarps) parts *= 2;
+    const int parts = min(32, (96 * d.sms + d.nclus - 1) / d.nclus);
     const long long warps = (long long)d.nclus * parts;
     k_pairs<R><<<(unsigned)((warps + PAIR_WARPS - 1) / PAIR_WARPS), PAIR_THREADS, 0, s>>>(d, parts);
 }

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
     d.dx[0] = m.dx[0]; d.dx[1] = m.dx[1];
     d.q[0] = m.q[0]; d.q[1] = m.q[1];
     d.qRest = m.qRest; d.vp = m.vp; d.stepLim = m.stepLim;
-    d.relA = m.relA; d.relB = m.relB; d.relCap = CAP;
+    d.relA = m.relA; d.relB = m.relB; d.relD = nullptr; d.relCap = CAP;
     if (g.numScenes <= SMALL_SCENES) {
         for (int s = t; s < g.numScenes; s += blockDim.x) m.sp[s] = g.sp[s];
         d.sp = m.sp;

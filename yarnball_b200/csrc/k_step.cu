@@ -251,171 +251,228 @@ __global__ void __launch_bounds__(NT, MINB) k_iter(Dev<R> d, int src) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Load-balanced variant of k_iter (one lane per vertex).  The contact lists of the block's
-// B segments are consecutive in the packed layout (slots base + f, f = 0 .. total - 1); every
-// thread takes contacts f = tid, tid + B, ... of that range, so a warp never waits for its
-// longest list, the partner ids and staged positions are read coalesced, and the partner
-// gathers of the whole block are in flight together.  Each thread writes its
-// contact's 18-value contribution to shared memory (four 16-byte and one 8-byte store); the
-// owning segment then adds its contacts in list order, so the result is deterministic.  The
-// rest (own terms, vertex solve, orientation update) is k_iter's.
-template <typename R, int NT, int MINB>
+// Load-balanced kernel (one lane per vertex), the default.  The contact lists of a block's B
+// segments are consecutive in the packed layout; the block works through them in two stages:
+//   * every warp tests a run of the contacts, one per lane, for being certainly out of range.
+//     More than half of the listed contacts are farther apart than the barrier reaches (the lists
+//     hold every pair within the detection radius); such a contact contributes exactly zero.
+//     No point pair of two segments can be closer than their distance at the start of the
+//     substep (from the list pass) less the largest relative displacement of their end points,
+//     so a contact with dist - max |dx_a - dx_b| > 2 radius + barrierThickness needs no
+//     closest points.  The bound is nearly tight, since neighbours move together: 56 % of the
+//     entries certified where 59 % are out of range (pile of 65,536 vertices, 12.4 contacts a
+//     segment), 59 of 65 % (uneven batch after 3 frames), 99 of 99 % (bundle of parallel yarns);
+//   * the others, queued in order, are evaluated NT at a time, one per thread; contributions go
+//     through shared memory and the owning thread adds its own in list order.
+// Both stages run on full warps, whatever the lengths of the lists, and a warp's long lists are
+// shared by the block.  Skipping a contact without the queue would save nothing, since nearly
+// every warp holds one in range.  Results are bit for bit those of evaluating every contact.  The
+// vertex's own terms are loaded and added after the loop (their inputs are not live across it).
+// Bound by issue (53 % of the slots) and by the latency of the gathers, at 24 warps an SM; with 32
+// (64 registers, spilled) the large batch takes 6.43 ms per substep and the small scenes 10-20 %
+// longer than with 24.  Measured, 8 launches, every contact evaluated -> now: 8.4M vertices with
+// 3.2 contacts 7.91 -> 6.69 ms, bundle of 100,352 vertices with 13.7 contacts 336 -> 171 us, pile
+// of 65,792 with 11.5 contacts 324 -> 285 us, of 262,144 with 10.6 contacts 898 -> 925 us.
+template <typename R>
+__device__ __forceinline__ R rel2(const V4<R>& a, const V4<R>& b) {
+    const R x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
+    return x * x + y * y + z * z;
+}
+
+template <typename R, int B, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
-    constexpr int B = NT;
     constexpr int CORE = B - 2;
     constexpr int NW = NT / 32;
-    const int t = threadIdx.x;
-    const int k = blockIdx.x * CORE - 1 + t;
+    constexpr int SPAN = 256;  // contacts a warp tests before the queue is worked off
+    static_assert(B <= 256 && B <= NT, "the owner byte of a packed contact names a slot of the block");
+    const unsigned FULL = 0xffffffffu;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int kb = blockIdx.x * CORE - 1, k = kb + t;
     const int n = d.n;
-    const bool valid = (k >= 0) && (k < n);
+    const bool owns = B == NT || t < B;  // the others only help with the contacts
+    const bool valid = owns && (k >= 0) && (k < n);
     const D2<R>* __restrict__ DX = d.dx[src];
     const V4<R>* __restrict__ QO = d.q[src];
 
-    __shared__ R sSeg[12][B];  // p0, e = p1 - p0, dx, dx1 of each slot's segment
-    // contributions of one chunk of contacts, double buffered, in 16-byte groups:
-    // (fa, fb.x) (fb.yz, Ha0-1) (Ha2-5) (Hb0-3), then (Hb4-5)
-    __shared__ V4<R> sCon4[2][4][B];
-    __shared__ R2<R> sCon2[2][B];
-    __shared__ int sOwn[2][B];     // owning slot of each contact of a chunk (double buffered)
-    __shared__ int sOff[B + 1];
+    __shared__ V4<R> sA[B], sB[B];  // (dx, e.x) and (dx1, e.y) of each slot's segment, e = p1 - p0
+    __shared__ R sEz[B];
     __shared__ int sScene[B];
-    __shared__ int sWarp[NW];
-    __shared__ unsigned sBase;
+    // contributions of NT contacts in 16-byte groups: (fa, fb.x) (fb.yz, Ha0-1) (Ha2-5) (Hb0-3),
+    // then (Hb4-5)
+    __shared__ V4<R> sCon4[4][NT];
+    __shared__ R2<R> sCon2[NT];
+    __shared__ int sQueue[NW][SPAN];  // contacts to evaluate: place in the block's lists | owner << 16
+    __shared__ int sCount[2][NW];  // (two, so that a warp ahead of the others overwrites none that is still read)
+    __shared__ short sFirst[B], sEnd[B];  // each owner's entries among those evaluated
 
-    // The contact loop runs first and accumulates from zero; the vertex's own terms (inertia,
-    // glue, stretch) are loaded and added after it, so their inputs are not live (in
-    // registers) across the loop.
     V3<R> fa(R(0)), fb(R(0));
     H3<R> Ha, Hb;
     Ha.zero(); Hb.zero();
-    int nc = 0, sc = 0;
-    if (t == 0) sBase = d.csrOff[k < 0 ? 0 : k];  // the block's first packed slot (k < n here)
-    {
-        V3<R> p0(R(0)), e(R(0)), dx(R(0)), dx1(R(0));
-        if (valid) {
-            // inputs of the vertex's own terms, used after the contact loop
-            prefetch_l1(d.vel + k);
-            prefetch_l1(QO + k);
-            prefetch_l1(d.qRest + k);
-            prefetch_l1(d.stepLim + k);
-            const uint32_t fl = d.vp[k].flags;
-            sc = scene_of(fl);
-            const D2<R> own = DX[k];
-            dx = xyz(own.a);
-            dx1 = xyz(own.b);
-            p0 = xyz(d.pos[k]);
-            if (fl & F_HAS_NEXT) {
-                e = xyz(d.pos[k + 1]) - p0;
-                unsigned off;
-                nc = contact_range(d, k, off);
-            }
-        }
-        sSeg[0][t] = p0.x; sSeg[1][t] = p0.y; sSeg[2][t] = p0.z;
-        sSeg[3][t] = e.x; sSeg[4][t] = e.y; sSeg[5][t] = e.z;
-        sSeg[6][t] = dx.x; sSeg[7][t] = dx.y; sSeg[8][t] = dx.z;
-        sSeg[9][t] = dx1.x; sSeg[10][t] = dx1.y; sSeg[11][t] = dx1.z;
+    int sc = 0;
+    bool sound = true;
+    const unsigned base = d.csrOff[max(kb, 0)];
+    int total = (int)(d.csrOff[min(kb + B, n)] - base);
+    if (valid) {
+        // inputs of the vertex's own terms, used after the contact loop
+        prefetch_l1(d.vel + k);
+        prefetch_l1(QO + k);
+        prefetch_l1(d.qRest + k);
+        prefetch_l1(d.stepLim + k);
+        const unsigned off = d.csrOff[k], end = d.csrOff[k + 1];
+        const V4<R> P = d.pos[k];
+        const V4<R> P1 = d.pos[min(k + 1, n - 1)];
+        const D2<R> own = DX[k];
+        sc = scene_of(d.vp[k].flags);
+        V4<R> w;
+        w.x = own.a.x; w.y = own.a.y; w.z = own.a.z; w.w = P1.x - P.x; sA[t] = w;
+        w.x = own.b.x; w.y = own.b.y; w.z = own.b.z; w.w = P1.y - P.y; sB[t] = w;
+        sEz[t] = P1.z - P.z;
         sScene[t] = sc;
+        sound = end >= off && end - off <= (unsigned)MAX_COLS && end <= d.csrCap;
     }
-    // block exclusive scan of the contact counts (the block's packed slots are base + offset)
-    {
-        const int lane = t & 31, w = t >> 5;
-        int x = nc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) sWarp[w] = x;
-        __syncthreads();
-        int wo = 0;
-        for (int i = 0; i < w; i++) wo += sWarp[i];
-        sOff[t] = wo + x - nc;
-        if (t == B - 1) sOff[B] = wo + x;
-        __syncthreads();
+    if (owns) {
+        sFirst[t] = 0;
+        sEnd[t] = 0;
     }
-    int total = sOff[B];
-    int myOff = sOff[t];
-    const unsigned base = sBase;
-    if (base > d.csrCap || d.csrCap - base < (unsigned)total) {  // only a packing the list pass reported as failed
-        total = 0;
-        myOff = 0;
-        nc = 0;
-    }
-    // Chunks of NT contacts, one per thread.  Each thread writes its own slot index over its
-    // contacts of the next chunk before the current chunk's barrier, which publishes it, and
-    // the contributions are double buffered: a buffer is written again only after the next
-    // chunk's barrier, which every thread reaches after summing it, so each chunk needs one
-    // barrier.
-    for (int g = myOff; g < min(myOff + nc, NT); g++) sOwn[0][g] = t;
-    __syncthreads();
-    int buf = 0;
-    // The partner id of this thread's contact is loaded one chunk ahead (after the previous
-    // chunk's barrier, before its summation), so a chunk starts with the partner gather.
-    int jn = 0;
-    if (t < total) jn = __ldg(d.csrCols + (base + t));
-    for (int b0 = 0; b0 < total; b0 += NT, buf ^= 1) {
-        const int f = b0 + t;
-        {
-            const int nb = b0 + NT;
-            const int g1 = min(myOff + nc, nb + NT);
-            for (int g = max(myOff, nb); g < g1; g++) sOwn[buf ^ 1][g - nb] = t;
-        }
-        V3<R> cfa(R(0)), cfb(R(0));
-        H3<R> cHa, cHb;
-        cHa.zero(); cHb.zero();
-        if (f < total && partner_ok(d, jn)) {
-            const int s = sOwn[buf][t];
-            const int j = jn;
-            const V3<R> sp0(sSeg[0][s], sSeg[1][s], sSeg[2][s]);
-            V3<R> r0, r1;
-            partner_rel(d, base + f, j, sp0, r0, r1);
-            const D2<R> pd = DX[j];
-            const V3<R> se(sSeg[3][s], sSeg[4][s], sSeg[5][s]);
-            const V3<R> sdx(sSeg[6][s], sSeg[7][s], sSeg[8][s]);
-            const V3<R> sdx1(sSeg[9][s], sSeg[10][s], sSeg[11][s]);
-            contact_term(se, sdx, sdx1, r0, r1, xyz(pd.a), xyz(pd.b), d.sp[sScene[s]], cfa, cHa, cfb, cHb);
-        }
-        {
-            V4<R> w;
-            w.x = cfa.x; w.y = cfa.y; w.z = cfa.z; w.w = cfb.x; sCon4[buf][0][t] = w;
-            w.x = cfb.y; w.y = cfb.z; w.z = cHa.d[0]; w.w = cHa.d[1]; sCon4[buf][1][t] = w;
-            w.x = cHa.d[2]; w.y = cHa.d[3]; w.z = cHa.d[4]; w.w = cHa.d[5]; sCon4[buf][2][t] = w;
-            w.x = cHb.d[0]; w.y = cHb.d[1]; w.z = cHb.d[2]; w.w = cHb.d[3]; sCon4[buf][3][t] = w;
-            R2<R> w2;
-            w2.x = cHb.d[4]; w2.y = cHb.d[5];
-            sCon2[buf][t] = w2;
-        }
-        __syncthreads();
-        {
-            // next chunk: partner id, and the staged partner positions into L1
-            const int fn = b0 + NT + t;
-            if (fn < total) {
-                const unsigned g = base + fn;
-                jn = __ldg(d.csrCols + g);
-                if (g < d.relCap) {
-                    prefetch_l1(d.relA + g);
-                    prefetch_l1(d.relB + g);
-                }
-            }
-        }
-        const int f0 = max(myOff, b0), f1 = min(myOff + nc, b0 + NT);
-        for (int g = f0; g < f1; g++) {
-            const int i = g - b0;
-            const V4<R> w0 = sCon4[buf][0][i], w1 = sCon4[buf][1][i], w2 = sCon4[buf][2][i], w3 = sCon4[buf][3][i];
-            const R2<R> w4 = sCon2[buf][i];
-            fa += V3<R>(w0.x, w0.y, w0.z);
-            fb += V3<R>(w0.w, w1.x, w1.y);
-            Ha.d[0] += w1.z; Ha.d[1] += w1.w;
-            Ha.d[2] += w2.x; Ha.d[3] += w2.y; Ha.d[4] += w2.z; Ha.d[5] += w2.w;
-            Hb.d[0] += w3.x; Hb.d[1] += w3.y; Hb.d[2] += w3.z; Hb.d[3] += w3.w;
-            Hb.d[4] += w4.x; Hb.d[5] += w4.y;
-        }
-    }
+    // ranges the packed arrays cannot hold (only after a list pass that reported a failure): the
+    // block's lists read as empty
+    if (!__syncthreads_and(sound)) total = 0;
 
-    // The halo exchange after the loop uses the contribution buffer the last chunk did not
-    // use (buf), viewed as 16 rows of B values: every thread finished reading it before the
-    // last chunk's barrier.
-    R (*rows)[B] = reinterpret_cast<R (*)[B]>(&sCon4[buf][0][0]);
+    int turn = 0;
+    for (int f00 = 0; f00 < total; f00 += NW * SPAN, turn ^= 1) {
+        // this warp's contacts: a whole number of steps of 32
+        const int share = (min(total - f00, NW * SPAN) + 32 * NW - 1) / (32 * NW) * 32;
+        const int fBeg = f00 + wp * share, fEnd = min(fBeg + share, total);
+        {
+            int qn = 0;  // queued contacts (identical in every lane)
+            // A lane's contact is looked up two steps ahead (partner id, owner, squared room) and
+            // its partner's iterate loaded one step ahead.
+            int j1 = -1, j2 = -1, s1 = 0, s2 = 0;
+            R room1 = R(0), room2 = R(0);
+            D2<R> p1;
+            auto look = [&](int f) {
+                j2 = -1;
+                if (f < fEnd) {
+                    const unsigned g = base + (unsigned)f;
+                    j2 = __ldg(d.csrCols + g);
+                    s2 = (int)__ldg(d.csrOwner + g);
+                    room2 = g < d.relCap ? d.relD[g] : R(-1);
+                    if (!partner_ok(d, j2)) j2 = -1;
+                }
+            };
+            look(fBeg + lane);
+            j1 = j2; s1 = s2; room1 = room2;
+            if (j1 >= 0) p1 = DX[j1];
+            look(fBeg + 32 + lane);
+            for (int f = fBeg + lane; f - lane < fEnd; f += 32) {
+                const int j = j1, s = (s1 - kb) & 255;
+                const R room = room1;
+                const D2<R> pd = p1;
+                j1 = j2; s1 = s2; room1 = room2;
+                if (j1 >= 0) p1 = DX[j1];
+                look(f + 64);
+                bool live = false;
+                if (j >= 0) {
+                    const V4<R> A = sA[s], Bq = sB[s];
+                    // room is negative for a contact in range from the start; a comparison with
+                    // something that is not a number keeps the contact
+                    live = !(rel2(A, pd.a) < room && rel2(A, pd.b) < room && rel2(Bq, pd.a) < room &&
+                             rel2(Bq, pd.b) < room);
+                }
+                const unsigned lives = __ballot_sync(FULL, live);
+                if (live) {
+                    sQueue[wp][qn + __popc(lives & lt)] = f | s << 16;
+                    const unsigned g = base + (unsigned)f;
+                    if (g < d.relCap) {
+                        prefetch_l1(d.relA + g);
+                        prefetch_l1(d.relB + g);
+                    }
+                }
+                qn += __popc(lives);
+            }
+            if (lane == 0) sCount[turn][wp] = qn;
+        }
+        __syncthreads();
+        int before[NW + 1];
+        before[0] = 0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) before[w + 1] = before[w] + sCount[turn][w];
+        const int lives = before[NW];
+        auto queued = [&](int i) {  // entry i of the warps' queues, one after the other
+            int w = 0, o = 0;
+#pragma unroll
+            for (int v = 1; v < NW; v++)
+                if (i >= before[v]) {
+                    w = v;
+                    o = before[v];
+                }
+            return sQueue[w][i - o];
+        };
+        for (int i0 = 0; i0 < lives; i0 += NT) {
+            const int i = i0 + t;
+            V3<R> cfa(R(0)), cfb(R(0));
+            H3<R> cHa, cHb;
+            cHa.zero(); cHb.zero();
+            if (i < lives) {
+                const int e = queued(i);
+                const int s = e >> 16;
+                if (t == 0 || queued(i - 1) >> 16 != s) sFirst[s] = (short)t;
+                if (t == NT - 1 || i + 1 == lives || queued(i + 1) >> 16 != s) sEnd[s] = (short)(t + 1);
+                const unsigned g = base + (unsigned)(e & 0xffff);
+                const int j = __ldg(d.csrCols + g);
+                const D2<R> pd = DX[j];
+                const V4<R> A = sA[s], Bq = sB[s];
+                V3<R> r0, r1;
+                if (g < d.relCap) {
+                    const V4<R> ra = d.relA[g];
+                    const R2<R> rb = d.relB[g];
+                    r0 = V3<R>(ra.x, ra.y, ra.z);
+                    r1 = V3<R>(ra.w, rb.x, rb.y);
+                } else {
+                    const V3<R> p0 = xyz(d.pos[kb + s]);
+                    r0 = xyz(d.pos[j]) - p0;
+                    r1 = xyz(d.pos[j + 1]) - p0;
+                }
+                contact_term(V3<R>(A.w, Bq.w, sEz[s]), xyz(A), xyz(Bq), r0, r1, xyz(pd.a), xyz(pd.b), d.sp[sScene[s]],
+                             cfa, cHa, cfb, cHb);
+                V4<R> w;
+                w.x = cfa.x; w.y = cfa.y; w.z = cfa.z; w.w = cfb.x; sCon4[0][t] = w;
+                w.x = cfb.y; w.y = cfb.z; w.z = cHa.d[0]; w.w = cHa.d[1]; sCon4[1][t] = w;
+                w.x = cHa.d[2]; w.y = cHa.d[3]; w.z = cHa.d[4]; w.w = cHa.d[5]; sCon4[2][t] = w;
+                w.x = cHb.d[0]; w.y = cHb.d[1]; w.z = cHb.d[2]; w.w = cHb.d[3]; sCon4[3][t] = w;
+                R2<R> w2;
+                w2.x = cHb.d[4]; w2.y = cHb.d[5];
+                sCon2[t] = w2;
+            }
+            __syncthreads();
+            if (owns) {
+                const int g1 = sEnd[t];
+                for (int g = sFirst[t]; g < g1; g++) {
+                    const V4<R> c0 = sCon4[0][g], c1 = sCon4[1][g], c2 = sCon4[2][g], c3 = sCon4[3][g];
+                    const R2<R> c4 = sCon2[g];
+                    fa += V3<R>(c0.x, c0.y, c0.z);
+                    fb += V3<R>(c0.w, c1.x, c1.y);
+                    Ha.d[0] += c1.z; Ha.d[1] += c1.w;
+                    Ha.d[2] += c2.x; Ha.d[3] += c2.y; Ha.d[4] += c2.z; Ha.d[5] += c2.w;
+                    Hb.d[0] += c3.x; Hb.d[1] += c3.y; Hb.d[2] += c3.z; Hb.d[3] += c3.w;
+                    Hb.d[4] += c4.x; Hb.d[5] += c4.y;
+                }
+                sFirst[t] = 0;
+                sEnd[t] = 0;
+            }
+            __syncthreads();
+        }
+    }
+    if (!owns) return;
+    auto sync_owners = [] {  // a barrier of the owning threads
+        if constexpr (B == NT) __syncthreads();
+        else if constexpr (B == 32) __syncwarp();
+        else asm volatile("bar.sync 1, %0;" ::"n"(B) : "memory");
+    };
+
+    // The halo exchange after the loop uses the contributions' memory, viewed as rows of B values.
+    R (*rows)[B] = reinterpret_cast<R (*)[B]>(&sCon4[0][0]);
     R (*sFb)[B] = rows;       // rows 0-2
     R (*sHb)[B] = rows + 3;   // rows 3-8
     R* sSL = rows[9];
@@ -425,22 +482,23 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
     R sl = yinf<R>();
     uint32_t flags = 0;
     R invMass = R(0), lRest = R(1), kStretch = R(0);
-    const V3<R> p0(sSeg[0][t], sSeg[1][t], sSeg[2][t]);
-    const V3<R> e(sSeg[3][t], sSeg[4][t], sSeg[5][t]);
-    const V3<R> dx(sSeg[6][t], sSeg[7][t], sSeg[8][t]);
+    V3<R> e(R(0)), dx(R(0));
     Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
     const SceneParams<R>* spp = d.sp;
     if (valid) {
         spp = &d.sp[sc];
-        add_own_terms(d, k, DX, QO, *spp, p0, e, dx, V3<R>(sSeg[9][t], sSeg[10][t], sSeg[11][t]), fa, Ha, fb, Hb,
-                      flags, invMass, lRest, kStretch, sl, q0);
+        const V4<R> A = sA[t], Bq = sB[t];
+        dx = xyz(A);
+        e = V3<R>(A.w, Bq.w, sEz[t]);
+        add_own_terms(d, k, DX, QO, *spp, xyz(d.pos[k]), e, dx, xyz(Bq), fa, Ha, fb, Hb, flags, invMass, lRest,
+                      kStretch, sl, q0);
     }
 
     sFb[0][t] = fb.x; sFb[1][t] = fb.y; sFb[2][t] = fb.z;
 #pragma unroll
     for (int q = 0; q < 6; q++) sHb[q][t] = Hb.d[q];
     sSL[t] = sl;
-    __syncthreads();
+    sync_owners();
 
     V3<R> dxn = dx;
     if (valid && t > 0) {
@@ -460,172 +518,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
     }
     sDX[0][t] = dxn.x; sDX[1][t] = dxn.y; sDX[2][t] = dxn.z;
     const bool core = valid && t >= 1 && t <= CORE;
-    __syncthreads();
-
-    if (core) {
-        const V3<R> dxb(sDX[0][t + 1], sDX[1][t + 1], sDX[2][t + 1]);
-        D2<R> o;
-        o.a = v4(dxn, R(0));
-        o.b = v4(k + 1 < n ? dxb : V3<R>(R(0)), R(0));
-        d.dx[src ^ 1][k] = o;
-        d.q[src ^ 1][k] = v4of(orientation_update(d, k, QO, flags, e, dxn, dxb, lRest, kStretch, q0));
-    }
-}
-
-// Warp-balanced variant of k_iter_bal: each warp flattens the contact lists of its own 32
-// vertices (warp scan) and processes them 32 at a time, so the contact loop needs no block
-// barrier and warps of one block proceed independently; per vertex the contributions are still
-// summed in list order.
-template <typename R, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_iter_wbal(Dev<R> d, int src) {
-    constexpr int B = NT;
-    constexpr int CORE = B - 2;
-    constexpr int NW = NT / 32;
-    const int t = threadIdx.x;
-    const int k = blockIdx.x * CORE - 1 + t;
-    const int n = d.n;
-    const bool valid = (k >= 0) && (k < n);
-    const D2<R>* __restrict__ DX = d.dx[src];
-    const V4<R>* __restrict__ QO = d.q[src];
-
-    __shared__ R sFb[3][B];
-    __shared__ R sHb[6][B];
-    __shared__ R sSL[B];
-    __shared__ R sDX[3][B];
-    __shared__ R sSeg[12][B];  // p0, e = p1 - p0, dx, dx1 of each slot's segment
-    __shared__ R sCon[18][B];  // contributions of one chunk of contacts
-    __shared__ int sOffW[NW][33];
-    __shared__ int sScene[B];
-    __shared__ unsigned sKOff[B];  // first packed slot of each slot's contacts
-
-    // The contact loop runs first and accumulates from zero; the vertex's own terms are
-    // loaded and added after it (their inputs are not live across the loop).
-    V3<R> fa(R(0)), fb(R(0));
-    H3<R> Ha, Hb;
-    Ha.zero(); Hb.zero();
-    int nc = 0, sc = 0;
-    unsigned kOff = 0;
-    {
-        V3<R> p0(R(0)), e(R(0)), dx(R(0)), dx1(R(0));
-        if (valid) {
-            const uint32_t fl = d.vp[k].flags;
-            sc = scene_of(fl);
-            const D2<R> own = DX[k];
-            dx = xyz(own.a);
-            dx1 = xyz(own.b);
-            p0 = xyz(d.pos[k]);
-            if (fl & F_HAS_NEXT) {
-                e = xyz(d.pos[k + 1]) - p0;
-                nc = contact_range(d, k, kOff);
-            }
-        }
-        sSeg[0][t] = p0.x; sSeg[1][t] = p0.y; sSeg[2][t] = p0.z;
-        sSeg[3][t] = e.x; sSeg[4][t] = e.y; sSeg[5][t] = e.z;
-        sSeg[6][t] = dx.x; sSeg[7][t] = dx.y; sSeg[8][t] = dx.z;
-        sSeg[9][t] = dx1.x; sSeg[10][t] = dx1.y; sSeg[11][t] = dx1.z;
-        sScene[t] = sc;
-        sKOff[t] = kOff;
-    }
-    // warp exclusive scan of the contact counts: each warp flattens its own 32 vertices
-    const int lane = t & 31, wp = t >> 5, w0 = wp << 5;
-    int incl = nc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    sOffW[wp][lane] = incl - nc;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (lane == 31) sOffW[wp][32] = total;
-    __syncwarp();
-    const int myOff = incl - nc;
-    for (int base = 0; base < total; base += 32) {
-        const int f = base + lane;
-        V3<R> cfa(R(0)), cfb(R(0));
-        H3<R> cHa, cHb;
-        cHa.zero(); cHb.zero();
-        if (f < total) {
-            int lo = 0, hi = 31;  // owner: the last lane of the warp whose offset is <= f
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (sOffW[wp][mid] <= f) lo = mid; else hi = mid - 1;
-            }
-            const int s = w0 + lo, c = f - sOffW[wp][lo];
-            const unsigned g = sKOff[s] + c;
-            const int j = __ldg(d.csrCols + g);
-            if (partner_ok(d, j)) {
-                const V3<R> sp0(sSeg[0][s], sSeg[1][s], sSeg[2][s]);
-                V3<R> r0, r1;
-                partner_rel(d, g, j, sp0, r0, r1);
-                const D2<R> pd = DX[j];
-                const V3<R> se(sSeg[3][s], sSeg[4][s], sSeg[5][s]);
-                const V3<R> sdx(sSeg[6][s], sSeg[7][s], sSeg[8][s]);
-                const V3<R> sdx1(sSeg[9][s], sSeg[10][s], sSeg[11][s]);
-                contact_term(se, sdx, sdx1, r0, r1, xyz(pd.a), xyz(pd.b), d.sp[sScene[s]], cfa, cHa, cfb, cHb);
-            }
-        }
-        sCon[0][t] = cfa.x; sCon[1][t] = cfa.y; sCon[2][t] = cfa.z;
-        sCon[3][t] = cfb.x; sCon[4][t] = cfb.y; sCon[5][t] = cfb.z;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            sCon[6 + q][t] = cHa.d[q];
-            sCon[12 + q][t] = cHb.d[q];
-        }
-        __syncwarp();
-        const int f0 = max(myOff, base), f1 = min(myOff + nc, base + 32);
-        for (int g = f0; g < f1; g++) {
-            const int i = w0 + g - base;
-            fa += V3<R>(sCon[0][i], sCon[1][i], sCon[2][i]);
-            fb += V3<R>(sCon[3][i], sCon[4][i], sCon[5][i]);
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                Ha.d[q] += sCon[6 + q][i];
-                Hb.d[q] += sCon[12 + q][i];
-            }
-        }
-        __syncwarp();
-    }
-
-    // the vertex's own terms (cosserat.cu:40-81)
-    R sl = yinf<R>();
-    uint32_t flags = 0;
-    R invMass = R(0), lRest = R(1), kStretch = R(0);
-    const V3<R> p0(sSeg[0][t], sSeg[1][t], sSeg[2][t]);
-    const V3<R> e(sSeg[3][t], sSeg[4][t], sSeg[5][t]);
-    const V3<R> dx(sSeg[6][t], sSeg[7][t], sSeg[8][t]);
-    Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
-    const SceneParams<R>* spp = d.sp;
-    if (valid) {
-        spp = &d.sp[sc];
-        add_own_terms(d, k, DX, QO, *spp, p0, e, dx, V3<R>(sSeg[9][t], sSeg[10][t], sSeg[11][t]), fa, Ha, fb, Hb,
-                      flags, invMass, lRest, kStretch, sl, q0);
-    }
-
-    sFb[0][t] = fb.x; sFb[1][t] = fb.y; sFb[2][t] = fb.z;
-#pragma unroll
-    for (int q = 0; q < 6; q++) sHb[q][t] = Hb.d[q];
-    sSL[t] = sl;
-    __syncthreads();
-
-    V3<R> dxn = dx;
-    if (valid && t > 0) {
-        if (flags & F_HAS_PREV) {
-            fa += V3<R>(sFb[0][t - 1], sFb[1][t - 1], sFb[2][t - 1]);
-            H3<R> hp;
-#pragma unroll
-            for (int q = 0; q < 6; q++) hp.d[q] = sHb[q][t - 1];
-            Ha.add(hp);
-            sl = ymin(sl, sSL[t - 1]);
-        }
-        if (invMass != R(0)) {
-            dxn = dx + spp->accel * solve3(Ha, fa);
-            const R l = len(dxn);
-            if (l > sl && l > R(0)) dxn *= sl / l;
-        }
-    }
-    sDX[0][t] = dxn.x; sDX[1][t] = dxn.y; sDX[2][t] = dxn.z;
-    const bool core = valid && t >= 1 && t <= CORE;
-    __syncthreads();
+    sync_owners();
 
     if (core) {
         const V3<R> dxb(sDX[0][t + 1], sDX[1][t + 1], sDX[2][t + 1]);
@@ -651,23 +544,35 @@ void launch_end(const Dev<R>& d, int finalBuf, bool copyQ, bool kahan, cudaStrea
 }
 
 // Newton iteration launch shapes: NT threads per block, T lanes per vertex, pipelined or not;
-// lanes = 0 selects a load-balanced kernel (one lane per vertex, flattened contact lists):
-// per block (pipe = 0) or per warp (pipe = 1).
+// lanes = 0 selects the load-balanced kernel (one lane per vertex, flattened contact lists; pipe
+// makes no difference to it).
 template <typename R>
 void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, cudaStream_t s) {
     if (d.n <= 0) return;
 #define YB_ITER(NT, T, MINB, P) \
     k_iter<R, NT, T, MINB, P><<<(d.n + (NT / T) - 3) / ((NT / T) - 2), NT, 0, s>>>(d, srcBuf)
-    if (lanes == 0 && pipe) {  // warp-balanced contact loop
-        if constexpr (sizeof(R) == 4)
-            k_iter_wbal<R, 128, 6><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
-        else
-            k_iter_wbal<R, 64, 4><<<(d.n + 61) / 62, 64, 0, s>>>(d, srcBuf);
-    } else if (lanes == 0) {  // block-balanced contact loop (shared memory bounds the block size)
-        if constexpr (sizeof(R) == 4)
-            k_iter_bal<R, 128, 7><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
-        else
-            k_iter_bal<R, 64, 4><<<(d.n + 61) / 62, 64, 0, s>>>(d, srcBuf);
+    if (lanes == 0) {
+        // Load-balanced kernel.  A block of 128 slots fills the chip from about 112k vertices on (6
+        // blocks of 126 vertices on 148 SMs).  Below, a launch lasts as long as one block's chain
+        // of steps, so small blocks of 32 slots get 3 or 7 warps that only help with the contacts,
+        // while the grid still is one wave.  Time of 8 launches, 128 slots against 32 slots with
+        // 256 (128) threads: 91 against 69 (69) us at 1,949 vertices, 62 against 38 (43) at
+        // 12,827, 285 against 342 (283) at 65,792, 171 against 358 (228) at 100,352.  FP64 build,
+        // 32 slots with 128 threads against 128 slots: 69 against 103 us at 1,949 vertices, 102
+        // against 153 at 12,827, 503 against 383 at 94,560.  The results are the same bit for bit.
+        if constexpr (sizeof(R) == 4) {
+            if (d.n <= 30 * 3 * d.sms)
+                k_iter_bal<R, 32, 256, 3><<<(d.n + 29) / 30, 256, 0, s>>>(d, srcBuf);
+            else if (d.n <= 30 * 6 * d.sms)
+                k_iter_bal<R, 32, 128, 6><<<(d.n + 29) / 30, 128, 0, s>>>(d, srcBuf);
+            else
+                k_iter_bal<R, 128, 128, 6><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
+        } else {
+            if (d.n <= 30 * 3 * d.sms)
+                k_iter_bal<R, 32, 128, 3><<<(d.n + 29) / 30, 128, 0, s>>>(d, srcBuf);
+            else
+                k_iter_bal<R, 128, 128, 3><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
+        }
     } else if (pipe) {
         if (lanes == 4) YB_ITER(256, 4, 2, true);
         else if (threads == 128) YB_ITER(128, 1, 4, true);

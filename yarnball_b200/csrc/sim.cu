@@ -274,6 +274,7 @@ SceneParams<R> scene_params_of(const yb_meta& m) {
     p.accel = (R)m.accelerationRatio;
     p.twoR = R(2) * (R)m.radius;
     p.invb = R(1) / (R)m.barrierThickness;
+    p.outOfRange = (p.twoR + (R)m.barrierThickness) * R(1.001);
     p.kCol = (R)m.kCollision * p.invb;
     p.fricK = (R)m.kFriction;
     p.fricMu = (R)m.frictionCoeff;
@@ -350,11 +351,13 @@ struct Engine : EngineBase {
         want((void**)&d.cols, sizeof(int) * n * MAX_COLS);
         want((void**)&d.relA, sizeof(V4<R>) * n * RELCAP);
         want((void**)&d.relB, sizeof(R2<R>) * n * RELCAP);
+        want((void**)&d.relD, sizeof(R) * n * RELCAP);
         // packed contacts: every list at its cap fits (slot indices are 32-bit)
         const size_t csrCap = std::min(n * (size_t)MAX_COLS, (size_t)0xffffffffu);
         const size_t listTiles = (n + LIST_THREADS - 1) / LIST_THREADS;
         want((void**)&d.csrOff, sizeof(unsigned) * (n + 1));
         want((void**)&d.csrCols, sizeof(int) * csrCap);
+        want((void**)&d.csrOwner, csrCap);
         want((void**)&d.listStatus, sizeof(unsigned long long) * (1 + listTiles));
         want((void**)&d.segs, sizeof(int) * n);
         want((void**)&spDev, sizeof(SceneParams<R>) * ns);
@@ -418,7 +421,7 @@ struct Engine : EngineBase {
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             for (int m = 0; m < 2; m++) d.travBlocks[m] = sms * traverse_blocks_per_sm<R>(m);
-            d.pairWarps = sms * 32;
+            d.sms = sms;
         }
         d.travPacket = S->travPacket;
         YB_CUDA(small_path_prepare<R>());  // a recycled batch may become small later
@@ -1538,7 +1541,7 @@ yb_status yb_autotune(yb_sim* S, int32_t* bestThreads, int32_t* bestLanes, int32
     if (!S) return YB_ERR_INVALID_ARGUMENT;
     if (!S->configured) return YB_ERR_NOT_CONFIGURED;
     static const int shapes[][3] = {{256, 1, 0}, {128, 1, 0}, {256, 2, 0}, {256, 4, 0}, {512, 4, 0}, {256, 8, 0},
-                                    {512, 8, 0}, {128, 1, 1}, {256, 1, 1}, {256, 4, 1}, {128, 0, 0}, {128, 0, 1}};
+                                    {512, 8, 0}, {128, 1, 1}, {256, 1, 1}, {256, 4, 1}, {128, 0, 0}};
     constexpr int NS = sizeof(shapes) / sizeof(shapes[0]);
     float best = INFINITY;
     int bt = S->iterThreads, bl = S->iterLanes, bp = S->iterPipe;
