@@ -66,6 +66,8 @@ struct alignas(sizeof(R) * 2) R2 {
 
 constexpr int RELCAP = 16;  // staged contacts: RELCAP x vertices slots in all (a contact past them is gathered)
 constexpr int LIST_THREADS = 128;  // vertices per block of the list pass (one packed-offset tile)
+constexpr int SMALL_TILE = 32;     // ... in a small simulation
+__host__ __device__ constexpr int list_tiles(int n) { return (n + SMALL_TILE - 1) / SMALL_TILE; }  // at most
 
 // Wide records are built only for the nodes the walk loads: those at an even depth below
 // their scene's root (a record's entries are grandchildren).  Depths come from pointer jumping
@@ -179,7 +181,8 @@ struct Dev {
     unsigned char* csrOwner;  // low byte of each packed contact's vertex
     unsigned csrCap;  // slots of csrCols
     unsigned relCap;  // slots of relA / relB
-    unsigned long long* listStatus;  // list pass: [0] tile ticket, [1 + tile] look-back status
+    unsigned long long* listStatus;  // list pass: [0] tile ticket, [1 + tile] look-back status;
+                                     // zero between substeps (k_end)
     int* segs;        // segment -> vertex index, ascending (scene-contiguous)
     const SceneParams<R>* sp;
     int* err;         // EW_COUNT ints
@@ -215,20 +218,49 @@ struct Dev {
     unsigned* sceneBox;   // 6 ordered-uint per scene: min xyz, max xyz of segment midpoints
 };
 
+// The kernels of a substep are launched with programmatic dependence: the grid of one may be set up
+// while the one before it runs.  Each begins with this wait for the grid before it to complete and
+// its writes to be visible, before it touches any memory; only then it lets the next one be set
+// up, so at most one grid waits at a time.  (No effect in a kernel launched the plain way.)
+__device__ __forceinline__ void after_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a kernel that begins with after_previous_kernel().
+template <typename... P, typename... A>
+void launch_dependent(void (*kernel)(P...), size_t blocks, unsigned threads, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // an error stays for the caller's cudaGetLastError
+}
+
 // Hint: bring the line holding p into L1 (no register is held until the data is used).
 __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 // --- kernel launchers (stream-ordered; no host synchronisation) ---
-template <typename R> void launch_init(const Dev<R>& d, cudaStream_t s);
+// clearLists: a detection follows; the contact counts are zeroed for it.
+template <typename R> void launch_init(const Dev<R>& d, bool clearLists, cudaStream_t s);
 template <typename R> void launch_end(const Dev<R>& d, int finalBuf, bool copyQ, bool kahan, cudaStream_t s);
 template <typename R> void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, cudaStream_t s);
 template <typename R> void launch_bvh_rebuild(const Dev<R>& d, cudaStream_t s, void* sortScratch, size_t sortScratchBytes, int keyBits);
 template <typename R> void launch_bvh_refit(const Dev<R>& d, cudaStream_t s);
-template <typename R> void launch_traverse(const Dev<R>& d, cudaStream_t s);  // + list sort + step limit (2 kernels)
+// The pair search, list sort and step limit (2 kernels); the contact counts are zero (launch_init) or
+// zeroed here.
+template <typename R> void launch_traverse(const Dev<R>& d, bool cleared, cudaStream_t s);
 template <typename R> int traverse_blocks_per_sm(int mode);  // resident traversal blocks per SM (persistent grid)
 template <typename R> void launch_lists_step_limit(const Dev<R>& d, cudaStream_t s);  // step limit over segments
+// After a list pass that no launch_end follows: its look-back status must be zero before the next.
+template <typename R> void reset_list_status(const Dev<R>& d, cudaStream_t s);
 // Segment, cluster and level boxes in curve order; the cluster-pair search; per-scene boxes.
 template <typename R> void launch_boxes(const Dev<R>& d, cudaStream_t s);
 template <typename R> void launch_pairs(const Dev<R>& d, cudaStream_t s);

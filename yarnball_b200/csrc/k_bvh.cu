@@ -606,7 +606,7 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
     }
 }
 
-// List pass, every substep, over tiles of LIST_THREADS consecutive vertices.  Per segment after
+// List pass, every substep, over tiles of B consecutive vertices (NT threads).  Per segment after
 // the broadphase: clamp and check the count, sort the list by partner id (fixed summation order
 // in the Newton iteration); with sortLists = 0 the lists are kept (substeps without detection,
 // collision.cu:121-172).  Then the lists of all vertices are packed in vertex order (csrOff,
@@ -614,7 +614,7 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
 // first slot by decoupled look-back over the tiles before it, 32 at a time (they hold smaller
 // tickets, so they are running or done; each wait is bounded and a timeout sets
 // IE_LIST_WAIT).  The tile's
-// contacts are then evaluated 128 at a time, one per thread: the packed partner id, the
+// contacts are then evaluated NT at a time, one per thread: the packed partner id, the
 // partner endpoints staged relative to p0 in the same slot, and the step-size limit
 // (collision.cu:121-159), of which each segment takes the minimum over its contacts in list
 // order (the minimum is exact, so this equals a per-segment loop).  The packed slots are
@@ -624,22 +624,23 @@ constexpr unsigned long long LS_AGG = 1ull << 62;
 constexpr unsigned long long LS_PRE = 2ull << 62;
 constexpr unsigned long long LS_VAL = (1ull << 62) - 1;
 
-template <typename R>
-__global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists) {
-    constexpr int B = LIST_THREADS;
+template <typename R, int B, int NT>
+__global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     __shared__ int sOff[B + 1];
     __shared__ int sWarp[B / 32];
     __shared__ int sTile;
     __shared__ unsigned long long sBase;
     __shared__ R sA0[3][B], sA1[3][B];
     __shared__ int sScene[B];
-    __shared__ R sLim[B];
+    __shared__ R sLim[NT];
+    after_previous_kernel();
     const int t = threadIdx.x;
+    const bool owns = B == NT || t < B;  // the others only help with the contacts
     if (t == 0) sTile = (int)atomicAdd(d.listStatus, 1ull);
     __syncthreads();
     const int tile = sTile;
     const int k = tile * B + t;
-    const bool inRange = k < d.n;
+    const bool inRange = owns && k < d.n;
     bool valid = false;  // k is a segment
     int nc = 0, sc = 0, rawCount = 0;
     V3<R> a0(R(0)), a1(R(0));
@@ -665,19 +666,21 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        if (lane == 31) sWarp[w] = x;
+        if (owns && lane == 31) sWarp[w] = x;
         __syncthreads();
-        int wo = 0;
-        for (int i = 0; i < w; i++) wo += sWarp[i];
-        sOff[t] = wo + x - nc;
-        if (t == B - 1) sOff[B] = wo + x;
+        if (owns) {
+            int wo = 0;
+            for (int i = 0; i < w; i++) wo += sWarp[i];
+            sOff[t] = wo + x - nc;
+            if (t == B - 1) sOff[B] = wo + x;
+        }
         __syncthreads();
     }
     // The tile's count is published before the sort, so that a later tile's look-back rarely
     // has to wait for it.
     volatile unsigned long long* st = d.listStatus + 1;
     if (t == 0) st[tile] = (tile == 0 ? LS_PRE : LS_AGG) | (unsigned long long)sOff[B];
-    if (sortLists) {
+    if (sortLists && owns) {
         // largest list of the warp (before the clamp), one atomic per warp
         int m = rawCount;
 #pragma unroll
@@ -685,9 +688,11 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
         if ((t & 31) == 0 && m) atomicMax(&d.err[EW_MAX_COLS], m);
         sort_list(d, valid ? k : -1, nc);
     }
-    sScene[t] = sc;
-    sA0[0][t] = a0.x; sA0[1][t] = a0.y; sA0[2][t] = a0.z;
-    sA1[0][t] = a1.x; sA1[1][t] = a1.y; sA1[2][t] = a1.z;
+    if (owns) {
+        sScene[t] = sc;
+        sA0[0][t] = a0.x; sA0[1][t] = a0.y; sA0[2][t] = a0.z;
+        sA1[0][t] = a1.x; sA1[1][t] = a1.y; sA1[2][t] = a1.z;
+    }
     // first packed slot of this tile: decoupled look-back by warp 0, 32 predecessors at a time
     // (lane l reads tile hi - l; the window ends at the nearest tile that holds a prefix)
     if (t < 32) {
@@ -736,7 +741,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
     __syncthreads();
     const unsigned long long base = sBase;
     const int total = sOff[B];
-    const int myOff = sOff[t];
+    const int myOff = owns ? sOff[t] : total;
     if (inRange) {
         d.csrOff[k] = (unsigned)(base + myOff);
         if (k == d.n - 1) d.csrOff[d.n] = (unsigned)(base + myOff + nc);
@@ -745,7 +750,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
     if (valid) m = step_limit_base(d, k, d.sp[sc]);
     int pens = 0;
     float dmin = INFINITY;
-    for (int b0 = 0; b0 < total; b0 += B) {
+    for (int b0 = 0; b0 < total; b0 += NT) {
         const int f = b0 + t;
         R lim = yinf<R>();
         if (f < total) {
@@ -773,7 +778,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_lists(Dev<R> d, int sortLists)
         }
         sLim[t] = lim;
         __syncthreads();
-        const int f0 = max(myOff, b0), f1 = min(myOff + nc, b0 + B);
+        const int f0 = max(myOff, b0), f1 = min(myOff + nc, b0 + NT);
         for (int g = f0; g < f1; g++) m = ymin(m, sLim[g - b0]);
         __syncthreads();
     }
@@ -957,7 +962,7 @@ void launch_bvh_reset(const Dev<R>& d, cudaStream_t s) {
 template <typename R>
 void launch_bvh_refit(const Dev<R>& d, cudaStream_t s) {
     if (d.nseg <= 0) return;
-    launch_boxes(d, s);  // also for bounds()
+    launch_boxes(d, s);  // by every walk, for bounds()
     if (d.travPacket == 2) return;
     // one segment: no internal node, but its query record is written
     if (d.nseg > 1) cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * (d.nseg - 1), s);
@@ -967,15 +972,28 @@ void launch_bvh_refit(const Dev<R>& d, cudaStream_t s) {
 
 template <typename R>
 void launch_lists(const Dev<R>& d, int sortLists, cudaStream_t s) {
-    const int tiles = (d.n + LIST_THREADS - 1) / LIST_THREADS;
-    cudaMemsetAsync(d.listStatus, 0, sizeof(unsigned long long) * (1 + (size_t)tiles), s);
-    k_lists<R><<<tiles, LIST_THREADS, 0, s>>>(d, sortLists);
+    // A tile's contacts are worked NT at a time between barriers.  While the chip is far from full a
+    // launch lasts as long as one tile's chain of steps, so small tiles get helper threads: the class
+    // of the pair search and this pass takes 28 -> 23 us at 1,949 vertices, 54 -> 46 us in the FP64
+    // build at 12,827, 145 -> 134 us and 232 -> 218 us at 65,792 and 100,352, but 335 -> 349 us at
+    // 262,144 and 450 -> 554 us at 1.0M (a tile's fixed steps outweigh its contacts).
+    const int tiles = (d.n + SMALL_TILE - 1) / SMALL_TILE;
+    if (tiles <= 24 * d.sms)
+        launch_dependent(k_lists<R, SMALL_TILE, 128>, tiles, 128, s, d, sortLists);
+    else
+        launch_dependent(k_lists<R, LIST_THREADS, LIST_THREADS>, (d.n + LIST_THREADS - 1) / LIST_THREADS, LIST_THREADS, s,
+                         d, sortLists);
 }
 
 template <typename R>
-void launch_traverse(const Dev<R>& d, cudaStream_t s) {
+void reset_list_status(const Dev<R>& d, cudaStream_t s) {
+    cudaMemsetAsync(d.listStatus, 0, sizeof(unsigned long long) * (1 + (size_t)list_tiles(d.n)), s);
+}
+
+template <typename R>
+void launch_traverse(const Dev<R>& d, bool cleared, cudaStream_t s) {
     if (d.nseg <= 0) return;
-    cudaMemsetAsync(d.numCols, 0, sizeof(int) * d.n, s);
+    if (!cleared) cudaMemsetAsync(d.numCols, 0, sizeof(int) * d.n, s);
     if (d.travPacket == 2) {
         launch_pairs(d, s);
     } else {
@@ -1018,9 +1036,11 @@ int traverse_blocks_per_sm(int mode) {  // resident blocks of the traversal kern
 }
 template int traverse_blocks_per_sm<float>(int);
 template int traverse_blocks_per_sm<double>(int);
-template void launch_traverse<float>(const Dev<float>&, cudaStream_t);
+template void launch_traverse<float>(const Dev<float>&, bool, cudaStream_t);
+template void reset_list_status<float>(const Dev<float>&, cudaStream_t);
+template void reset_list_status<double>(const Dev<double>&, cudaStream_t);
 template void launch_lists_step_limit<float>(const Dev<float>&, cudaStream_t);
 template void launch_lists_step_limit<double>(const Dev<double>&, cudaStream_t);
-template void launch_traverse<double>(const Dev<double>&, cudaStream_t);
+template void launch_traverse<double>(const Dev<double>&, bool, cudaStream_t);
 
 }  // namespace yb

@@ -54,6 +54,7 @@ constexpr int BOX_THREADS = 1024;
 
 template <typename R>
 __global__ void __launch_bounds__(BOX_THREADS) k_boxes(Dev<R> d, const int* __restrict__ sortedVals) {
+    after_previous_kernel();
     __shared__ float4 sLo[32], sHi[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int s = d.l1Scene[blockIdx.x];
@@ -167,6 +168,7 @@ __device__ __noinline__ void pairs_filter(const Dev<R>& d, const PairShare& sh, 
 
 template <typename R>
 __global__ void __launch_bounds__(PAIR_THREADS, 8) k_pairs(const __grid_constant__ Dev<R> d, int parts) {
+    after_previous_kernel();
     const unsigned FULL = 0xffffffffu;
     __shared__ PairShare share[PAIR_WARPS];
     const int lane = threadIdx.x & 31;
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(32) k_scene_box(Dev<R> d, float* out) {
 
 template <typename R>
 void launch_boxes(const Dev<R>& d, cudaStream_t s) {
-    if (d.nl1 > 0) k_boxes<R><<<d.nl1, BOX_THREADS, 0, s>>>(d, d.vals[0]);
+    if (d.nl1 > 0) launch_dependent(k_boxes<R>, d.nl1, BOX_THREADS, s, d, d.vals[0]);
 }
 
 template <typename R>
@@ -325,7 +327,7 @@ void launch_pairs(const Dev<R>& d, cudaStream_t s) {
     if (d.nclus <= 0) return;
     const int parts = min(32, (96 * d.sms + d.nclus - 1) / d.nclus);
     const long long warps = (long long)d.nclus * parts;
-    k_pairs<R><<<(unsigned)((warps + PAIR_WARPS - 1) / PAIR_WARPS), PAIR_THREADS, 0, s>>>(d, parts);
+    launch_dependent(k_pairs<R>, (size_t)((warps + PAIR_WARPS - 1) / PAIR_WARPS), PAIR_THREADS, s, d, parts);
 }
 
 template <typename R>

@@ -18,9 +18,11 @@
 namespace yb {
 
 template <typename R>
-__global__ void __launch_bounds__(256) k_init(Dev<R> d) {
+__global__ void __launch_bounds__(256) k_init(Dev<R> d, int clearLists) {
+    after_previous_kernel();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
+    if (clearLists) d.numCols[i] = 0;
     init_vertex(d, i);
 }
 
@@ -29,8 +31,10 @@ __global__ void __launch_bounds__(256) k_init(Dev<R> d) {
 // also stores the start-of-substep velocity as lastVel (iteration.cu:19-20).
 template <typename R>
 __global__ void __launch_bounds__(256) k_end(Dev<R> d, int fb, int copyQ, int kahan) {
+    after_previous_kernel();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.n) return;
+    if (i <= list_tiles(d.n)) d.listStatus[i] = 0ull;  // for the next list pass (n is 3 or more)
     end_vertex(d, i, fb, copyQ, kahan);
 }
 
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
     constexpr int NW = NT / 32;
     constexpr int SPAN = 256;  // contacts a warp tests before the queue is worked off
     static_assert(B <= 256 && B <= NT, "the owner byte of a packed contact names a slot of the block");
+    after_previous_kernel();
     const unsigned FULL = 0xffffffffu;
     const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -532,15 +537,15 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
 
 // ---------------------------------------------------------------------------------------
 template <typename R>
-void launch_init(const Dev<R>& d, cudaStream_t s) {
+void launch_init(const Dev<R>& d, bool clearLists, cudaStream_t s) {
     if (d.n <= 0) return;
-    k_init<R><<<(d.n + 255) / 256, 256, 0, s>>>(d);
+    launch_dependent(k_init<R>, (d.n + 255) / 256, 256, s, d, clearLists ? 1 : 0);
 }
 
 template <typename R>
 void launch_end(const Dev<R>& d, int finalBuf, bool copyQ, bool kahan, cudaStream_t s) {
     if (d.n <= 0) return;
-    k_end<R><<<(d.n + 255) / 256, 256, 0, s>>>(d, finalBuf, copyQ ? 1 : 0, kahan ? 1 : 0);
+    launch_dependent(k_end<R>, (d.n + 255) / 256, 256, s, d, finalBuf, copyQ ? 1 : 0, kahan ? 1 : 0);
 }
 
 // Newton iteration launch shapes: NT threads per block, T lanes per vertex, pipelined or not;
@@ -560,16 +565,22 @@ void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, 
         // 12,827, 285 against 342 (283) at 65,792, 171 against 358 (228) at 100,352.  FP64 build,
         // 32 slots with 128 threads against 128 slots: 69 against 103 us at 1,949 vertices, 102
         // against 153 at 12,827, 503 against 383 at 94,560.  The results are the same bit for bit.
+        // A grid that is most of one wave is launched the plain way: set up while the one before
+        // runs, its blocks would land on the SMs with the most room left instead of evenly (285
+        // against 315 us at 65,792 vertices).  Elsewhere the early set-up gains: 67 -> 59 us at
+        // 1,949, 103 -> 91 us FP64 at 12,827, 842 -> 827 us at 1.0M.
         if constexpr (sizeof(R) == 4) {
             if (d.n <= 30 * 3 * d.sms)
-                k_iter_bal<R, 32, 256, 3><<<(d.n + 29) / 30, 256, 0, s>>>(d, srcBuf);
+                launch_dependent(k_iter_bal<R, 32, 256, 3>, (d.n + 29) / 30, 256, s, d, srcBuf);
             else if (d.n <= 30 * 6 * d.sms)
-                k_iter_bal<R, 32, 128, 6><<<(d.n + 29) / 30, 128, 0, s>>>(d, srcBuf);
-            else
+                launch_dependent(k_iter_bal<R, 32, 128, 6>, (d.n + 29) / 30, 128, s, d, srcBuf);
+            else if (d.n <= 126 * 6 * d.sms)
                 k_iter_bal<R, 128, 128, 6><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
+            else
+                launch_dependent(k_iter_bal<R, 128, 128, 6>, (d.n + 125) / 126, 128, s, d, srcBuf);
         } else {
             if (d.n <= 30 * 3 * d.sms)
-                k_iter_bal<R, 32, 128, 3><<<(d.n + 29) / 30, 128, 0, s>>>(d, srcBuf);
+                launch_dependent(k_iter_bal<R, 32, 128, 3>, (d.n + 29) / 30, 128, s, d, srcBuf);
             else
                 k_iter_bal<R, 128, 128, 3><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
         }
@@ -589,8 +600,8 @@ void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, 
 #undef YB_ITER
 }
 
-template void launch_init<float>(const Dev<float>&, cudaStream_t);
-template void launch_init<double>(const Dev<double>&, cudaStream_t);
+template void launch_init<float>(const Dev<float>&, bool, cudaStream_t);
+template void launch_init<double>(const Dev<double>&, bool, cudaStream_t);
 template void launch_end<float>(const Dev<float>&, int, bool, bool, cudaStream_t);
 template void launch_end<double>(const Dev<double>&, int, bool, bool, cudaStream_t);
 template void launch_iter<float>(const Dev<float>&, int, int, int, int, cudaStream_t);

@@ -354,7 +354,7 @@ struct Engine : EngineBase {
         want((void**)&d.relD, sizeof(R) * n * RELCAP);
         // packed contacts: every list at its cap fits (slot indices are 32-bit)
         const size_t csrCap = std::min(n * (size_t)MAX_COLS, (size_t)0xffffffffu);
-        const size_t listTiles = (n + LIST_THREADS - 1) / LIST_THREADS;
+        const size_t listTiles = (size_t)list_tiles((int)n);
         want((void**)&d.csrOff, sizeof(unsigned) * (n + 1));
         want((void**)&d.csrCols, sizeof(int) * csrCap);
         want((void**)&d.csrOwner, csrCap);
@@ -431,6 +431,7 @@ struct Engine : EngineBase {
         static const int kInfBits = 0x7f800000;  // EW_MIN_DIST starts at +inf
         YB_CUDA(cudaMemcpyAsync(d.err + EW_MIN_DIST, &kInfBits, sizeof(int), cudaMemcpyHostToDevice, S->stream));
         YB_CUDA(cudaMemsetAsync(d.numCols, 0, sizeof(int) * n, S->stream));
+        YB_CUDA(cudaMemsetAsync(d.listStatus, 0, sizeof(unsigned long long) * (1 + listTiles), S->stream));
         // no packed contacts until the first list pass (a Newton launch before it reads none)
         YB_CUDA(cudaMemsetAsync(d.csrOff, 0, sizeof(unsigned) * (n + 1), S->stream));
         YB_CUDA(cudaMemsetAsync(d.lastVel, 0, sizeof(V4<R>) * n, S->stream));
@@ -805,7 +806,7 @@ struct Engine : EngineBase {
     uint64_t enqueue_substep(bool detect, bool rebuild, unsigned long long* slots = nullptr) override {
         cudaStream_t st = S->stream;
         uint64_t k = 0;
-        launch_init(d, st); k++;
+        launch_init(d, detect && d.nseg > 0, st); k++;
         if (detect && d.nseg > 0) {
             if (rebuild) {  // the schedule rebuilds first after any path that did not use the tree
                 launch_bvh_rebuild(d, st, sortScratch, sortBytes, keyBits);
@@ -815,7 +816,7 @@ struct Engine : EngineBase {
                 launch_bvh_refit(d, st);
                 k += refit_launches();
             }
-            launch_traverse(d, st); k += 2;
+            launch_traverse(d, true, st); k += 2;
         } else {
             launch_lists_step_limit(d, st); k++;
         }
@@ -1040,7 +1041,7 @@ struct Engine : EngineBase {
         };
         const int I = num_itr();
         mark(0);
-        launch_init(d, st); launches[0]++;
+        launch_init(d, detect && d.nseg > 0, st); launches[0]++;
         if (detect && d.nseg > 0) {
             if (rebuild || !bvhBuilt) {
                 mark(1);
@@ -1053,7 +1054,7 @@ struct Engine : EngineBase {
                 launches[2] += refit_launches();
             }
             mark(3);
-            launch_traverse(d, st); launches[3] += 2;
+            launch_traverse(d, true, st); launches[3] += 2;
         } else {
             mark(4);
             launch_lists_step_limit(d, st); launches[4]++;
@@ -1128,7 +1129,7 @@ struct Engine : EngineBase {
     uint64_t debug_phases(int mask, int& buf) override {
         cudaStream_t st = S->stream;
         uint64_t k = 0;
-        if (mask & 1) { launch_init(d, st); k++; buf = 0; }
+        if (mask & 1) { launch_init(d, false, st); k++; buf = 0; }
         if ((mask & 6) && d.nseg > 0) {
             if ((mask & 2) || !bvhBuilt) {  // a refit needs a tree
                 launch_bvh_rebuild(d, st, sortScratch, sortBytes, keyBits);
@@ -1138,10 +1139,15 @@ struct Engine : EngineBase {
                 launch_bvh_refit(d, st);
                 k += refit_launches();
             }
-            launch_traverse(d, st);
+            launch_traverse(d, false, st);
+            reset_list_status(d, st);
             k += 2;
         }
-        if (mask & 8) { launch_lists_step_limit(d, st); k++; }
+        if (mask & 8) {
+            launch_lists_step_limit(d, st);
+            reset_list_status(d, st);
+            k++;
+        }
         if (mask & 16) { launch_iter(d, buf, S->iterThreads, S->iterLanes, S->iterPipe, st); buf ^= 1; k++; }
         if (mask & 32) { launch_end(d, buf, buf != 0, sizeof(R) == 4, st); buf = 0; k++; }
         return k;
