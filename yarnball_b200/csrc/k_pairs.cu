@@ -18,8 +18,8 @@
 // dependent loads per segment; a walk is paid once per 32 segments.
 //
 // Measured (B200, per detection, refit + walk of the BVH before -> boxes + pairs): 8.4M vertices
-// in 269 scenes, 3.2 contacts a segment: 1.27 + 3.9 ms -> 0.17 + 2.6 ms; one pile of 65,792
-// vertices, 11.5 contacts: 49 + 280 us -> 10 + 89 us; a swatch of 1,949 vertices: 32 + 78 us -> 7 + 12 us.
+// in 269 scenes, 3.2 contacts a segment: 1.27 + 3.9 ms -> 0.17 + 2.2 ms; one pile of 65,792
+// vertices, 11.5 contacts: 49 + 280 us -> 10 + 75 us; a swatch of 1,949 vertices: 32 + 78 us -> 7 + 12 us.
 //
 // Boxes are kept in single precision in both builds, rounded outwards in the FP64 one: a box
 // may only be too large, and what it lets through the filter decides.
@@ -126,13 +126,12 @@ __global__ void __launch_bounds__(BOX_THREADS) k_boxes(Dev<R> d, const int* __re
 // shared memory and every lane tests its own segment against them in a loop (two broadcast
 // 16-byte reads and six compares a test), collecting the hits in a bit mask.  Hits go through a
 // queue of the warp, so that the separately rounded narrow-phase test runs on 32 pairs at once.
-// Bound by issue and latency (ncu, a million vertices: half of the issue slots busy at 38 % of
-// the warps).  `parts` makes 96 warps for every SM, three times what an SM holds, since the
-// clusters' work is uneven: the class of this kernel and the list pass takes 330 / 232 / 222 us
+// Bound by issue and latency.  `parts` makes 96 warps for every SM, three times what an SM holds, since the
+// clusters' work is uneven (blocks of 4 warps: this kernel and the list pass take 330 / 232 / 222 us
 // with 32 / 96 / 192 warps per SM on a bundle of 100,352 vertices, 144 / 146 / 163 us on a pile
-// of 65,792 and 365 / 342 / 361 us on one of 262,144 (every part repeats the walk).
-constexpr int PAIR_THREADS = 128;
-constexpr int PAIR_WARPS = PAIR_THREADS / 32;
+// of 65,792 and 365 / 342 / 361 us on one of 262,144; every part repeats the walk).
+constexpr int PAIR_THREADS = 32;  // a warp to a block: the clusters' work is uneven, and a block holds its
+                                  // place on the SM until its last warp is done (128 threads: 20 % longer)
 
 struct PairShare {
     float4 lo[32], hi[32];
@@ -144,7 +143,7 @@ struct PairShare {
 // registers would otherwise be held back from every warp of the search.
 template <typename R>
 __device__ __noinline__ void pairs_filter(const Dev<R>& d, const PairShare& sh, int first, int m, int s) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x;
     if (lane < m) {
         const int a = sh.qx[first + lane], b = sh.qy[first + lane];
         const int x = min(a, b), y = max(a, b);
@@ -167,14 +166,13 @@ __device__ __noinline__ void pairs_filter(const Dev<R>& d, const PairShare& sh, 
 }
 
 template <typename R>
-__global__ void __launch_bounds__(PAIR_THREADS, 8) k_pairs(const __grid_constant__ Dev<R> d, int parts) {
+__global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constant__ Dev<R> d, int parts) {
     after_previous_kernel();
     const unsigned FULL = 0xffffffffu;
-    __shared__ PairShare share[PAIR_WARPS];
-    const int lane = threadIdx.x & 31;
+    __shared__ PairShare sh;
+    const int lane = threadIdx.x;
     const unsigned lt = (1u << lane) - 1u;
-    PairShare& sh = share[threadIdx.x >> 5];
-    const int gw = (int)((blockIdx.x * (unsigned)PAIR_THREADS + threadIdx.x) >> 5);
+    const int gw = (int)blockIdx.x;
     const int ci = gw / parts, part = gw - ci * parts;
     if (ci >= d.nclus) return;
     const int s = d.clusScene[ci];
@@ -326,8 +324,7 @@ template <typename R>
 void launch_pairs(const Dev<R>& d, cudaStream_t s) {
     if (d.nclus <= 0) return;
     const int parts = min(32, (96 * d.sms + d.nclus - 1) / d.nclus);
-    const long long warps = (long long)d.nclus * parts;
-    launch_dependent(k_pairs<R>, (size_t)((warps + PAIR_WARPS - 1) / PAIR_WARPS), PAIR_THREADS, s, d, parts);
+    launch_dependent(k_pairs<R>, (size_t)d.nclus * parts, PAIR_THREADS, s, d, parts);
 }
 
 template <typename R>
