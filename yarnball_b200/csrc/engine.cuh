@@ -272,11 +272,13 @@ void launch_pin_drive(const Dev<R>& d, const float4* init, const unsigned char* 
                       cudaStream_t s);  // scene roots := empty
 
 // One block advances a small simulation (n <= 256 vertices) through `steps` substeps in one launch.
+// It takes the scenes' parameters from `params` (page-locked host memory; null: they are in d.sp)
+// and leaves them in d.sp, and writes the error words to errOut (page-locked host memory) as well.
 template <typename R> bool small_path_fits(const Dev<R>& d);
 template <typename R> cudaError_t small_path_prepare();  // once per device, before the first launch
 template <typename R>
-void launch_small(const Dev<R>& d, int steps, int numItr, unsigned long long step0, int detectionPeriod, bool kahan,
-                  cudaStream_t s);
+void launch_small(const Dev<R>& d, const SceneParams<R>* params, int* errOut, int steps, int numItr,
+                  unsigned long long step0, int detectionPeriod, bool kahan, cudaStream_t s);
 
 // Radix sort of (u64 key, int value) pairs, ascending by the low `bits` key bits, stable.
 // keys/vals ping-pong between [0] and [1]; the result lands in buffer (passes & 1).

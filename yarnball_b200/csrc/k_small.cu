@@ -69,8 +69,8 @@ __device__ __forceinline__ void small_min(double* at, double v) {
 
 template <typename R>
 __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
-    k_small(const __grid_constant__ Dev<R> g, int steps, int numItr, unsigned long long step0, int detectionPeriod,
-            int kahan) {
+    k_small(const __grid_constant__ Dev<R> g, const SceneParams<R>* params, int* errOut, int steps, int numItr,
+            unsigned long long step0, int detectionPeriod, int kahan) {
     constexpr int CT = SmallShare<R>::CT, CAP = SmallShare<R>::CAP;
     const unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char raw[];
@@ -87,9 +87,20 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
     d.q[0] = m.q[0]; d.q[1] = m.q[1];
     d.qRest = m.qRest; d.vp = m.vp; d.stepLim = m.stepLim;
     d.relA = m.relA; d.relB = m.relB; d.relD = nullptr; d.relCap = CAP;
-    if (g.numScenes <= SMALL_SCENES) {
-        for (int s = t; s < g.numScenes; s += blockDim.x) m.sp[s] = g.sp[s];
-        d.sp = m.sp;
+    {
+        // word by word, so that a whole warp reads host memory at once
+        static_assert(sizeof(SceneParams<R>) % 8 == 0, "parameters are copied by 8 bytes");
+        const int words = g.numScenes * (int)(sizeof(SceneParams<R>) / 8);
+        const bool here = g.numScenes <= SMALL_SCENES;
+        const unsigned long long* from = reinterpret_cast<const unsigned long long*>(params ? params : g.sp);
+        unsigned long long* keep = reinterpret_cast<unsigned long long*>(const_cast<SceneParams<R>*>(g.sp));
+        unsigned long long* to = reinterpret_cast<unsigned long long*>(m.sp);
+        for (int i = t; i < words; i += blockDim.x) {
+            const unsigned long long w = from[i];
+            if (params) keep[i] = w;
+            if (here) to[i] = w;
+        }
+        if (here) d.sp = m.sp;
     }
     uint32_t fl0 = 0;
     int nc = 0;
@@ -370,6 +381,8 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
         g.err[EW_WARNING] = 2;
     }
     if (dmin < INFINITY) atomicMin(&g.err[EW_MIN_DIST], __float_as_int(dmin));
+    __syncthreads();
+    if (t < EW_COUNT) errOut[t] = __ldcg(g.err + t);
 }
 
 template <typename R>
@@ -384,17 +397,18 @@ cudaError_t small_path_prepare() {
 }
 
 template <typename R>
-void launch_small(const Dev<R>& d, int steps, int numItr, unsigned long long step0, int detectionPeriod, bool kahan,
-                  cudaStream_t s) {
+void launch_small(const Dev<R>& d, const SceneParams<R>* params, int* errOut, int steps, int numItr,
+                  unsigned long long step0, int detectionPeriod, bool kahan, cudaStream_t s) {
     if (d.n <= 0 || steps <= 0) return;
     const int threads = (d.n + 31) / 32 * 32 + SmallShare<R>::CT;
-    k_small<R><<<1, threads, sizeof(SmallShare<R>), s>>>(d, steps, numItr, step0, detectionPeriod, kahan ? 1 : 0);
+    k_small<R><<<1, threads, sizeof(SmallShare<R>), s>>>(d, params, errOut, steps, numItr, step0, detectionPeriod, kahan ? 1 : 0);
 }
 
 #define YB_INST(R)                                                                                            \
     template bool small_path_fits<R>(const Dev<R>&);                                                          \
     template cudaError_t small_path_prepare<R>();                                                             \
-    template void launch_small<R>(const Dev<R>&, int, int, unsigned long long, int, bool, cudaStream_t);
+    template void launch_small<R>(const Dev<R>&, const SceneParams<R>*, int*, int, int, unsigned long long, int, bool, \
+                                  cudaStream_t);
 YB_INST(float)
 YB_INST(double)
 
