@@ -12,9 +12,9 @@
 // shortened and split over roles:
 //   * `vt` vertex threads (one vertex each) and CT contact threads.  In a Newton iteration the
 //     contact threads evaluate the contacts, CT at a time and one per thread, while the vertex
-//     threads evaluate inertia, glue and stretch, then sum the contributions in list order; the
-//     next iteration's contacts start as soon as the new displacements are known, beside the
-//     orientation update;
+//     threads evaluate inertia, glue and stretch, then sum the contributions in list order and
+//     solve, beside the bending gradients of the contact threads; the next iteration's contacts
+//     start as soon as the new displacements are known, beside the orientation update;
 //   * the pair search tests all padded boxes, every pair of vertices once, spread over all
 //     threads; hits go through a queue per warp so that the exact narrow phase runs on 32 pairs
 //     at once;
@@ -52,7 +52,7 @@ struct SmallShare {
     R2<R> relB[CAP];
     int pack[CAP];         // owner << 16 | partner
     R halo[10][SMALL_VERTS];  // fb, Hb and the step limit of each segment
-    R newDx[3][SMALL_VERTS];
+    V4<R> bend[SMALL_VERTS];  // gradient of each segment's bending terms
     float4 boxLo[SMALL_VERTS], boxHi[SMALL_VERTS];
     unsigned adj[SMALL_VERTS][SMALL_WORDS];
     int queue[WARPS][64];
@@ -259,7 +259,18 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
         if (valid && !(seg && d.sp[sc].useStepLimit)) m.stepLim[k] = yinf<R>();
 
         const int chunks = (total + CT - 1) / CT;
+        const bool bendHere = chunks == 0;  // else the contact threads have no time to spare
         int buf = 0;
+        OwnTerms<R> own;
+        own.flags = 0;
+        own.invMass = R(0);
+        own.sl = yinf<R>();
+        V3<R> p0(R(0)), e(R(0));
+        if (valid) {
+            own = own_terms(d, k, d.sp[sc]);
+            p0 = xyz(m.pos[k]);
+            if (seg) e = xyz(m.pos[k + 1]) - p0;
+        }
         for (int it = 0; it < numItr; it++) {
             const int src = it & 1;
             const D2<R>* DX = m.dx[src];
@@ -269,15 +280,15 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                 if (u < 0 || f >= total) return;
                 const int e = f < CAP ? m.pack[f] : g.csrCols[f];
                 const int a = e >> 16, o = e & 0xffff;
-                const V3<R> p0 = xyz(m.pos[a]);
+                const V3<R> a0 = xyz(m.pos[a]);
                 V3<R> r0, r1;
-                partner_rel(d, (unsigned)f, o, p0, r0, r1);
-                const D2<R> own = DX[a], pd = DX[o];
+                partner_rel(d, (unsigned)f, o, a0, r0, r1);
+                const D2<R> ad = DX[a], pd = DX[o];
                 V3<R> fa(R(0)), fb(R(0));
                 H3<R> Ha, Hb;
                 Ha.zero();
                 Hb.zero();
-                contact_term(xyz(m.pos[a + 1]) - p0, xyz(own.a), xyz(own.b), r0, r1, xyz(pd.a), xyz(pd.b),
+                contact_term(xyz(m.pos[a + 1]) - a0, xyz(ad.a), xyz(ad.b), r0, r1, xyz(pd.a), xyz(pd.b),
                              d.sp[scene_of(m.vp[a].flags)], fa, Ha, fb, Hb);
                 V4<R> w;
                 w.x = fa.x; w.y = fa.y; w.z = fa.z; w.w = fb.x; m.con4[to][0][u] = w;
@@ -292,24 +303,28 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
             H3<R> Ha, Hb;
             Ha.zero();
             Hb.zero();
-            R sl = yinf<R>();
-            uint32_t flags = 0;
-            R invMass = R(0), lRest = R(1), kStretch = R(0);
+            R sl = own.sl;
             Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
-            V3<R> p0(R(0)), e(R(0)), dx(R(0));
+            V3<R> dx(R(0));
             if (chunks) evaluate(0, buf);
             if (valid) {
-                const D2<R> own = DX[k];
-                dx = xyz(own.a);
-                p0 = xyz(m.pos[k]);
-                if (seg) e = xyz(m.pos[k + 1]) - p0;
-                add_own_terms(d, k, DX, QO, d.sp[sc], p0, e, dx, xyz(own.b), fa, Ha, fb, Hb, flags, invMass, lRest,
-                              kStretch, sl, q0);
+                const D2<R> ad = DX[k];
+                dx = xyz(ad.a);
+                q0 = qof(QO[k]);
+                add_own_terms(d, own, DX, d.sp[sc].D, p0, e, dx, xyz(ad.b), q0, fa, Ha, fb, Hb);
             }
-            for (int c = 0; c < chunks; c++, buf ^= 1) {
-                __syncthreads();  // chunk c is evaluated, and chunk c - 1 summed
-                if (c + 1 < chunks) evaluate(c + 1, buf ^ 1);
-                if (vertexWarp) {
+            for (int c = 0; c < max(chunks, 1); c++, buf ^= 1) {
+                // chunk c is evaluated, chunk c - 1 summed, and the rotors are those of the last iteration
+                __syncthreads();
+                if (c + 1 < chunks)
+                    evaluate(c + 1, buf ^ 1);
+                else if (bendHere)
+                    for (int i = t - vt; i < n; i += CT)
+                        if (i >= 0) {
+                            const uint32_t fl = m.vp[i].flags;
+                            if (turns(fl)) m.bend[i] = v4of(bending_gradient(d, i, QO, fl, qof(QO[i])));
+                        }
+                if (vertexWarp && c < chunks) {
                     const int f1 = min(off + nc, (c + 1) * CT) - c * CT;
                     for (int i = max(off - c * CT, 0); i < f1; i++) {
                         const V4<R> w0 = m.con4[buf][0][i], w1 = m.con4[buf][1][i], w2 = m.con4[buf][2][i],
@@ -332,7 +347,7 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                 m.halo[9][k] = sl;
                 asm volatile("bar.sync 1, %0;" ::"r"(vt) : "memory");  // the vertex threads only
                 if (valid) {
-                    if (flags & F_HAS_PREV) {
+                    if (own.flags & F_HAS_PREV) {
                         fa += V3<R>(m.halo[0][k - 1], m.halo[1][k - 1], m.halo[2][k - 1]);
                         H3<R> hp;
 #pragma unroll
@@ -340,7 +355,7 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                         Ha.add(hp);
                         sl = ymin(sl, m.halo[9][k - 1]);
                     }
-                    if (invMass != R(0)) {
+                    if (own.invMass != R(0)) {
                         dxn = dx + d.sp[sc].accel * solve3(Ha, fa);
                         const R l = len(dxn);
                         if (l > sl && l > R(0)) dxn *= sl / l;
@@ -352,9 +367,11 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                 }
             }
             __syncthreads();
-            if (valid)
-                m.q[src ^ 1][k] = v4of(orientation_update(d, k, QO, flags, e, dxn, xyz(m.dx[src ^ 1][k].b), lRest,
-                                                          kStretch, q0));
+            if (valid) {
+                if (turns(own.flags))
+                    q0 = turned(q0, bendHere ? qof(m.bend[k]) : bending_gradient(d, k, QO, own.flags, q0), e, dxn, xyz(m.dx[src ^ 1][k].b), own.invl, own.kStretch);
+                m.q[src ^ 1][k] = v4of(q0);
+            }
         }
         if (numItr & 1) {
             __syncthreads();  // neighbours still read q[0], which end_vertex overwrites

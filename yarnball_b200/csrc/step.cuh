@@ -6,6 +6,7 @@
 //   contact_term          cosseratItr's contact loop, sim/cosserat.cu:92-148
 //   add_own_terms         cosseratItr's inertia, glue and stretch terms, sim/cosserat.cu:40-81
 //   orientation_update    quaternionLambdaItr, sim/cosserat.cu:209-253
+//   own_terms, bending_gradient, turned: parts of the last two
 #pragma once
 #include "detect.cuh"
 
@@ -259,6 +260,115 @@ __device__ __forceinline__ Q<R> orientation_update(const Dev<R>& d, int k, const
         }
     }
     return qn;
+}
+
+// ---------------------------------------------------------------------------------------
+// The own terms and the orientation update in parts, for the one-block kernel, which forms once per
+// substep what its iterations share and evaluates the bending terms beside the solve: the same
+// expressions as above (in the multi-block kernel the parts cost 1.5 % over the functions above).
+
+// What the vertex's own terms need beside the iterates; the same in every iteration of a substep.
+// inertia and y are set for free vertices, invl and ks for segments.
+template <typename R>
+struct OwnTerms {
+    uint32_t flags;
+    int cid;
+    R lRest, kStretch, invMass, sl;
+    R inertia;   // m / h^2
+    V3<R> y;     // inertial target h v + h^2 g, formed here
+    R invl, ks;  // 1 / lRest, kStretch / lRest
+};
+
+template <typename R>
+__device__ __forceinline__ OwnTerms<R> own_terms(const Dev<R>& d, int k, const SceneParams<R>& sp) {
+    OwnTerms<R> w;
+    const VP<R> vp = d.vp[k];
+    w.flags = vp.flags;
+    w.cid = vp.cid;
+    w.lRest = vp.lRest;
+    w.kStretch = vp.kStretch;
+    w.invMass = d.pos[k].w;
+    if (w.invMass != R(0)) {
+        const V4<R> v = d.vel[k];
+        const R hh = sp.hh;
+        w.y = V3<R>(sp.h * v.x + hh * sp.gx, sp.h * v.y + hh * sp.gy, sp.h * v.z + hh * sp.gz);
+        w.inertia = R(1) / (w.invMass * hh);
+    }
+    w.sl = yinf<R>();
+    if (w.flags & F_HAS_NEXT) {
+        w.sl = d.stepLim[k];
+        w.invl = R(1) / w.lRest;
+        w.ks = w.kStretch * w.invl;
+    }
+    return w;
+}
+
+// The vertex's own terms added to force and Hessian sums that already hold its contacts: inertia
+// (H = m/h^2, f = m/h^2 (y - dx)), the glue spring to a connected vertex, and the stretch-shear
+// coupling of segment k to its orientation (its other endpoint's share in fb, Hb).
+template <typename R>
+__device__ __forceinline__ void add_own_terms(const Dev<R>& d, const OwnTerms<R>& w, const D2<R>* __restrict__ DX, R D,
+                                              const V3<R>& p0, const V3<R>& e, const V3<R>& dx, const V3<R>& dx1,
+                                              const Q<R>& q0, V3<R>& fa, H3<R>& Ha, V3<R>& fb, H3<R>& Hb) {
+    if (w.invMass != R(0)) {
+        Ha.add_diag(w.inertia);
+        fa += w.inertia * (w.y - dx);
+    }
+    if (w.cid >= 0) {
+        const R stiff = R(40);
+        const V3<R> pc = xyz(d.pos[w.cid]);
+        const V3<R> dc = xyz(DX[w.cid].a);
+        fa -= stiff * ((p0 - pc) + (dx - dc) + D * dx);
+        Ha.add_diag(stiff * (R(1) + D));
+    }
+    if (w.flags & F_HAS_NEXT) {
+        const V3<R> c = (e + (dx1 - dx)) * w.invl - qrotate(q0, V3<R>(R(1), R(0), R(0)));
+        R dd = w.ks * w.invl;
+        fa += w.ks * c - (D * dd) * dx;
+        fb += -w.ks * c - (D * dd) * dx1;
+        dd *= R(1) + D;
+        Ha.add_diag(dd);
+        Hb.add_diag(dd);
+    }
+}
+
+// Whether segment k's orientation is updated, and the gradient b of its bending terms from the
+// previous iteration's rotors (quaternionLambdaItr, cosserat.cu:209-253).
+__device__ __forceinline__ bool turns(uint32_t flags) { return !(flags & F_FIX_ORI) && (flags & F_HAS_NEXT); }
+
+template <typename R>
+__device__ __forceinline__ Q<R> bending_gradient(const Dev<R>& d, int k, const V4<R>* __restrict__ QO, uint32_t flags,
+                                                 const Q<R>& q0) {
+    Q<R> b = qmk(R(0), R(0), R(0), R(0));
+    if (flags & F_HAS_PREV) {
+        const Q<R> qr = qof(d.qRest[k - 1]);
+        const Q<R> qq = qof(QO[k - 1]);
+        const R s = qdot(qmul(qinv(qq), q0), qr) > R(0) ? R(1) : R(-1);
+        b = qadd(b, qscale(s, qmul(qq, qr)));
+    }
+    if (flags & F_HAS_NEXT_ORI) {
+        const Q<R> qr = qof(d.qRest[k]);
+        const Q<R> qq = qof(QO[k + 1]);
+        const R s = qdot(qmul(qinv(q0), qq), qr) > R(0) ? R(1) : R(-1);
+        b = qadd(b, qscale(s, qmul(qq, qinv(qr))));
+    }
+    return b;
+}
+
+// Closed-form orientation update of segment k (the same function of the reference) from the new
+// iterates of its endpoints (dxn, dxb) and the gradient b.  A single-segment yarn has no bending
+// neighbours (b = 0): the closed form is 0/0 there (the reference produces NaN); its orientation
+// is kept.
+template <typename R>
+__device__ __forceinline__ Q<R> turned(const Q<R>& q0, const Q<R>& b, const V3<R>& e, const V3<R>& dxn,
+                                       const V3<R>& dxb, R invl, R kStretch) {
+    V3<R> v = (e + (dxb - dxn)) * invl;
+    v *= R(-2) * kStretch;
+    const R bl = qlen(b);
+    if (!(bl > R(0))) return q0;
+    const R lambda = len(v) + bl;
+    const Q<R> vb1 = qmul(qmul(qmk(v, R(0)), b), qmk(R(1), R(0), R(0), R(0)));
+    return qnormalize(qadd(vb1, qscale(lambda, b)));
 }
 
 }  // namespace yb
