@@ -12,6 +12,10 @@ max position error / max displacement <= 1e-4, the bar of the FP32 build everywh
 1e-9 x segment length in the FP64 build.  The tangle of 256 vertices runs in the FP64 build: it
 amplifies rounding (two orders of summation in single precision differ by up to 2.6e-4 of the
 displacement within the frame).
+
+Newton kernels: a scene alone takes the one of its size, in a batch of its copies that of the batch's;
+the states are bit for bit the same, on either side of the sizes where the kernel changes, with
+connected vertices, and with more contacts in a block than its helping warps take at once.
 """
 import numpy as np
 import pytest
@@ -142,3 +146,31 @@ def test_one_block_sizes_vs_fp64_oracle(name):
         assert sim.debug_contacts()[0].sum() > 2560
     sim.close()
     orc.close()
+
+
+ALONE = {
+    # name: (yarn lengths, cube, glue, precision)
+    "257": ([128, 129], 0.02, False, "fp32"),
+    "1949_glued": ([31] * 62 + [27], 0.02, True, "fp32"),
+    "dense": ([125] * 16, 0.015, False, "fp32"),
+    "8880": ([80] * 111, 0.04, False, "fp32"),
+    "8881": ([83] * 107, 0.04, False, "fp32"),
+    "257_fp64": ([128, 129], 0.02, False, "fp64"),
+    "4440_fp64": ([40] * 111, 0.03, True, "fp64"),
+    "4441_fp64": ([4441 // 3] * 2 + [4441 - 2 * (4441 // 3)], 0.03, False, "fp64"),
+}
+
+
+@pytest.mark.parametrize("name", list(ALONE))
+def test_newton_kernels_of_all_sizes_agree_bit_for_bit(name):
+    lens, cube, glue, precision = ALONE[name]
+    sim = _walks(lens, 11, cube, glue, precision)
+    copies = 30000 // sim.numVerts + 1  # past the sizes of the small blocks
+    batch = Sim.gather([(sim, 0)] * copies)
+    for s in (sim, batch):
+        s.advance(4 * H)
+    a, b = sim.read_state_f64(), batch.read_state_f64()
+    for x, y in zip(a, b):
+        for c in (0, copies - 1):
+            o = batch.sceneOffsets[c]
+            assert np.array_equal(x, y[o:o + sim.numVerts])

@@ -536,6 +536,254 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
 }
 
 // ---------------------------------------------------------------------------------------
+// The same iteration for small simulations, where a launch lasts as long as one block's chain of
+// dependent steps (some 10k cycles) and most of the chip's issue slots are free.  A block has 32
+// slots: warp 0 owns them, the other warps work on the contacts in the same two stages.  While they
+// evaluate, the owners form the costly parts of their own terms and the bending gradients, which
+// k_iter_bal does after the sums; halo values pass between lanes instead of shared memory.  Every sum
+// has k_iter_bal's order and terms, and the parts formed early are chosen so that the compiler fuses
+// the rest alike: the results are the same bit for bit.
+// Needs 128 registers (FP64 242): at 80, where six blocks of 128 threads fit an SM, 430 bytes spill and
+// the launch takes 6 to 20 % longer than k_iter_bal's.  Measured, us per iteration within a substep, k_iter_bal with
+// 32 slots -> this kernel, swatches of 780 / 1,949 / 4,032 / 7,900 vertices: 6.2 / 6.2 / 6.4 / 6.7 ->
+// 5.1 / 5.4 / 5.4 / 5.6; FP64 build, 780 / 1,949 / 4,032 vertices: 7.2 / 7.0 / 7.6 -> 6.1 / 6.0 / 6.4.
+// 192 and 160 threads (112, 96 registers) gain nothing, 384 threads no more than 256.
+template <typename R, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_iter_small(Dev<R> d, int src) {
+    after_previous_kernel();
+    constexpr int CORE = 30;
+    constexpr int HELP = NT - 32, HW = HELP / 32;
+    constexpr int STEPS = 2, SPAN = 32 * STEPS;  // contacts a warp tests before the queue is worked off
+    const unsigned FULL = 0xffffffffu;
+    const int t = threadIdx.x, lane = t & 31, h = t - 32, wp = h >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const bool owns = t < 32;
+    const int kb = blockIdx.x * CORE - 1, k = kb + lane;
+    const int n = d.n;
+    const bool valid = owns && k >= 0 && k < n;
+    const D2<R>* __restrict__ DX = d.dx[src];
+    const V4<R>* __restrict__ QO = d.q[src];
+
+    __shared__ V4<R> sA[32], sB[32];  // (dx, e.x) and (dx1, e.y) of each slot's segment, e = p1 - p0
+    __shared__ R sEz[32];
+    __shared__ int sScene[32];
+    __shared__ V4<R> sCon4[4][HELP];  // contributions, grouped as in k_iter_bal
+    __shared__ R2<R> sCon2[HELP];
+    __shared__ int sQueue[HW][SPAN];  // contacts to evaluate: place in the block's lists | owner << 16
+    __shared__ int sCount[2][HW];
+    __shared__ short sFirst[32], sEnd[32];  // each owner's entries among those evaluated
+
+    const unsigned base = d.csrOff[max(kb, 0)];
+    int total = (int)(d.csrOff[min(kb + 32, n)] - base);
+    int sc = 0;
+    bool sound = true;
+    V3<R> p0(R(0)), e(R(0)), dx(R(0)), dx1(R(0));
+    int fBeg = 0, fEnd = 0;  // a helper warp's contacts
+    int j[STEPS], s[STEPS];
+    R room[STEPS];
+    D2<R> pd[STEPS];
+    auto load = [&](int f00) {
+        const int share = (min(total - f00, HW * SPAN) + 32 * HW - 1) / (32 * HW) * 32;
+        fBeg = f00 + wp * share;
+        fEnd = min(fBeg + share, total);
+#pragma unroll
+        for (int q = 0; q < STEPS; q++) {
+            const int f = fBeg + 32 * q + lane;
+            const unsigned g = base + (unsigned)f;
+            j[q] = -1;
+            if (f < fEnd && g < d.csrCap) {
+                j[q] = __ldg(d.csrCols + g);
+                s[q] = ((int)__ldg(d.csrOwner + g) - kb) & 31;
+                room[q] = g < d.relCap ? d.relD[g] : R(-1);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < STEPS; q++) {
+            if (!partner_ok(d, j[q])) j[q] = -1;
+            if (j[q] >= 0) pd[q] = DX[j[q]];
+        }
+    };
+    if (valid) {
+        // inputs of the vertex's own terms, used later
+        prefetch_l1(d.vel + k);
+        prefetch_l1(QO + k);
+        prefetch_l1(d.qRest + k);
+        prefetch_l1(d.stepLim + k);
+        const unsigned off = d.csrOff[k], end = d.csrOff[k + 1];
+        const V4<R> P = d.pos[k];
+        const V4<R> P1 = d.pos[min(k + 1, n - 1)];
+        const D2<R> own = DX[k];
+        sc = scene_of(d.vp[k].flags);
+        p0 = xyz(P);
+        e = xyz(P1) - p0;
+        dx = xyz(own.a);
+        dx1 = xyz(own.b);
+        sA[lane] = v4(dx, e.x);
+        sB[lane] = v4(dx1, e.y);
+        sEz[lane] = e.z;
+        sScene[lane] = sc;
+        sound = end >= off && end - off <= (unsigned)MAX_COLS && end <= d.csrCap;
+    } else if (!owns) {
+        load(0);
+    }
+    if (owns) {
+        sFirst[lane] = 0;
+        sEnd[lane] = 0;
+    }
+    if (!__syncthreads_and(sound)) total = 0;  // as in k_iter_bal
+
+    V3<R> fa(R(0)), fb(R(0));
+    H3<R> Ha, Hb;
+    Ha.zero(); Hb.zero();
+    OwnParts<R> w;
+    Q<R> bend = qmk(R(0), R(0), R(0), R(0));
+    bool prepared = false;
+    auto prepare = [&] {
+        prepared = true;
+        if (!valid) return;
+        w = own_parts(d, k, QO, d.sp[sc]);
+        const uint32_t fl = d.vp[k].flags;
+        if (turns(fl)) bend = bending_gradient(d, k, QO, fl, w.q0);
+    };
+    int turn = 0;
+    for (int f00 = 0; f00 < total; f00 += HW * SPAN, turn ^= 1) {
+        if (!owns) {
+            int qn = 0;  // queued contacts (identical in every lane)
+#pragma unroll
+            for (int q = 0; q < STEPS; q++) {
+                const int f = fBeg + 32 * q + lane;
+                bool live = false;
+                if (j[q] >= 0) {
+                    const V4<R> A = sA[s[q]], Bq = sB[s[q]];
+                    live = !(rel2(A, pd[q].a) < room[q] && rel2(A, pd[q].b) < room[q] && rel2(Bq, pd[q].a) < room[q] &&
+                             rel2(Bq, pd[q].b) < room[q]);
+                }
+                const unsigned lives = __ballot_sync(FULL, live);
+                if (live) {
+                    sQueue[wp][qn + __popc(lives & lt)] = f | s[q] << 16;
+                    const unsigned g = base + (unsigned)f;
+                    if (g < d.relCap) {
+                        prefetch_l1(d.relA + g);
+                        prefetch_l1(d.relB + g);
+                    }
+                }
+                qn += __popc(lives);
+            }
+            if (lane == 0) sCount[turn][wp] = qn;
+        }
+        __syncthreads();
+        int before[HW + 1];
+        before[0] = 0;
+#pragma unroll
+        for (int v = 0; v < HW; v++) before[v + 1] = before[v] + sCount[turn][v];
+        const int lives = before[HW];
+        auto queued = [&](int i) {  // entry i of the warps' queues, one after the other
+            int v = 0, o = 0;
+#pragma unroll
+            for (int u = 1; u < HW; u++)
+                if (i >= before[u]) {
+                    v = u;
+                    o = before[u];
+                }
+            return sQueue[v][i - o];
+        };
+        for (int i0 = 0; i0 < lives; i0 += HELP) {
+            const int i = i0 + h;
+            if (owns) {
+                if (!prepared) prepare();
+            } else if (i < lives) {
+                const int en = queued(i);
+                const int so = en >> 16;
+                if (h == 0 || queued(i - 1) >> 16 != so) sFirst[so] = (short)h;
+                if (h == HELP - 1 || i + 1 == lives || queued(i + 1) >> 16 != so) sEnd[so] = (short)(h + 1);
+                const unsigned g = base + (unsigned)(en & 0xffff);
+                const int jo = __ldg(d.csrCols + g);
+                const D2<R> po = DX[jo];
+                const V4<R> A = sA[so], Bq = sB[so];
+                V3<R> r0, r1;
+                if (g < d.relCap) {
+                    const V4<R> ra = d.relA[g];
+                    const R2<R> rb = d.relB[g];
+                    r0 = V3<R>(ra.x, ra.y, ra.z);
+                    r1 = V3<R>(ra.w, rb.x, rb.y);
+                } else {
+                    const V3<R> a0 = xyz(d.pos[kb + so]);
+                    r0 = xyz(d.pos[jo]) - a0;
+                    r1 = xyz(d.pos[jo + 1]) - a0;
+                }
+                V3<R> cfa(R(0)), cfb(R(0));
+                H3<R> cHa, cHb;
+                cHa.zero(); cHb.zero();
+                contact_term(V3<R>(A.w, Bq.w, sEz[so]), xyz(A), xyz(Bq), r0, r1, xyz(po.a), xyz(po.b), d.sp[sScene[so]],
+                             cfa, cHa, cfb, cHb);
+                V4<R> c;
+                c.x = cfa.x; c.y = cfa.y; c.z = cfa.z; c.w = cfb.x; sCon4[0][h] = c;
+                c.x = cfb.y; c.y = cfb.z; c.z = cHa.d[0]; c.w = cHa.d[1]; sCon4[1][h] = c;
+                c.x = cHa.d[2]; c.y = cHa.d[3]; c.z = cHa.d[4]; c.w = cHa.d[5]; sCon4[2][h] = c;
+                c.x = cHb.d[0]; c.y = cHb.d[1]; c.z = cHb.d[2]; c.w = cHb.d[3]; sCon4[3][h] = c;
+                R2<R> c2;
+                c2.x = cHb.d[4]; c2.y = cHb.d[5];
+                sCon2[h] = c2;
+            }
+            __syncthreads();
+            if (owns) {
+                const int g1 = sEnd[lane];
+                for (int g = sFirst[lane]; g < g1; g++) {
+                    const V4<R> c0 = sCon4[0][g], c1 = sCon4[1][g], c2 = sCon4[2][g], c3 = sCon4[3][g];
+                    const R2<R> c4 = sCon2[g];
+                    fa += V3<R>(c0.x, c0.y, c0.z);
+                    fb += V3<R>(c0.w, c1.x, c1.y);
+                    Ha.d[0] += c1.z; Ha.d[1] += c1.w;
+                    Ha.d[2] += c2.x; Ha.d[3] += c2.y; Ha.d[4] += c2.z; Ha.d[5] += c2.w;
+                    Hb.d[0] += c3.x; Hb.d[1] += c3.y; Hb.d[2] += c3.z; Hb.d[3] += c3.w;
+                    Hb.d[4] += c4.x; Hb.d[5] += c4.y;
+                }
+                sFirst[lane] = 0;
+                sEnd[lane] = 0;
+            }
+            if (i0 + HELP < lives || f00 + HW * SPAN < total) __syncthreads();
+        }
+        if (!owns && f00 + HW * SPAN < total) load(f00 + HW * SPAN);
+    }
+    if (!owns) return;
+    if (!prepared) prepare();
+    uint32_t flags = 0;
+    R invMass = R(0), lRest = R(1), kStretch = R(0), sl = yinf<R>();
+    Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
+    if (valid)
+        add_own_terms(d, k, DX, QO, d.sp[sc], p0, e, dx, dx1, fa, Ha, fb, Hb, flags, invMass, lRest, kStretch, sl, q0,
+                      &w);
+
+    // the previous segment's shares (cosserat.cu:175-205)
+    V3<R> pf(__shfl_up_sync(FULL, fb.x, 1), __shfl_up_sync(FULL, fb.y, 1), __shfl_up_sync(FULL, fb.z, 1));
+    H3<R> ph;
+#pragma unroll
+    for (int q = 0; q < 6; q++) ph.d[q] = __shfl_up_sync(FULL, Hb.d[q], 1);
+    const R psl = __shfl_up_sync(FULL, sl, 1);
+    V3<R> dxn = dx;
+    if (valid && lane > 0) {
+        if (flags & F_HAS_PREV) {
+            fa += pf;
+            Ha.add(ph);
+            sl = ymin(sl, psl);
+        }
+        if (invMass != R(0)) {
+            dxn = dx + d.sp[sc].accel * solve3(Ha, fa);
+            const R l = len(dxn);
+            if (l > sl && l > R(0)) dxn *= sl / l;
+        }
+    }
+    const V3<R> dxb(__shfl_down_sync(FULL, dxn.x, 1), __shfl_down_sync(FULL, dxn.y, 1), __shfl_down_sync(FULL, dxn.z, 1));
+    if (valid && lane >= 1 && lane <= CORE) {
+        D2<R> o;
+        o.a = v4(dxn, R(0));
+        o.b = v4(k + 1 < n ? dxb : V3<R>(R(0)), R(0));
+        d.dx[src ^ 1][k] = o;
+        d.q[src ^ 1][k] = v4of(turns(flags) ? turned(q0, bend, e, dxn, dxb, w.invl, kStretch) : q0);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 template <typename R>
 void launch_init(const Dev<R>& d, bool clearLists, cudaStream_t s) {
     if (d.n <= 0) return;
@@ -557,32 +805,40 @@ void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, 
 #define YB_ITER(NT, T, MINB, P) \
     k_iter<R, NT, T, MINB, P><<<(d.n + (NT / T) - 3) / ((NT / T) - 2), NT, 0, s>>>(d, srcBuf)
     if (lanes == 0) {
-        // Load-balanced kernel.  A block of 128 slots fills the chip from about 112k vertices on (6
+        // Load-balanced kernels.  A block of 128 slots fills the chip from about 112k vertices on (6
         // blocks of 126 vertices on 148 SMs).  Below, a launch lasts as long as one block's chain
         // of steps, so small blocks of 32 slots get 3 or 7 warps that only help with the contacts,
         // while the grid still is one wave.  Time of 8 launches, 128 slots against 32 slots with
         // 256 (128) threads: 91 against 69 (69) us at 1,949 vertices, 62 against 38 (43) at
         // 12,827, 285 against 342 (283) at 65,792, 171 against 358 (228) at 100,352.  FP64 build,
         // 32 slots with 128 threads against 128 slots: 69 against 103 us at 1,949 vertices, 102
-        // against 153 at 12,827, 503 against 383 at 94,560.  The results are the same bit for bit.
+        // against 153 at 12,827, 503 against 383 at 94,560.
+        // k_iter_small wins while its blocks, two to an SM (FP64: one) for their registers, are one
+        // wave; past that its second wave costs more: 6.9 against 9.7 us an iteration at 11,875
+        // vertices, FP64 8.0 against 11.1 at 7,900.  The results are the same bit for bit.
         // A grid that is most of one wave is launched the plain way: set up while the one before
         // runs, its blocks would land on the SMs with the most room left instead of evenly (285
         // against 315 us at 65,792 vertices).  Elsewhere the early set-up gains: 67 -> 59 us at
         // 1,949, 103 -> 91 us FP64 at 12,827, 842 -> 827 us at 1.0M.
+        const size_t small = (d.n + 29) / 30, large = (d.n + 125) / 126;
         if constexpr (sizeof(R) == 4) {
-            if (d.n <= 30 * 3 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 256, 3>, (d.n + 29) / 30, 256, s, d, srcBuf);
+            if (d.n <= 30 * 2 * d.sms)
+                launch_dependent(k_iter_small<R, 256, 2>, small, 256, s, d, srcBuf);
+            else if (d.n <= 30 * 3 * d.sms)
+                launch_dependent(k_iter_bal<R, 32, 256, 3>, small, 256, s, d, srcBuf);
             else if (d.n <= 30 * 6 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 128, 6>, (d.n + 29) / 30, 128, s, d, srcBuf);
+                launch_dependent(k_iter_bal<R, 32, 128, 6>, small, 128, s, d, srcBuf);
             else if (d.n <= 126 * 6 * d.sms)
-                k_iter_bal<R, 128, 128, 6><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
+                k_iter_bal<R, 128, 128, 6><<<large, 128, 0, s>>>(d, srcBuf);
             else
-                launch_dependent(k_iter_bal<R, 128, 128, 6>, (d.n + 125) / 126, 128, s, d, srcBuf);
+                launch_dependent(k_iter_bal<R, 128, 128, 6>, large, 128, s, d, srcBuf);
         } else {
-            if (d.n <= 30 * 3 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 128, 3>, (d.n + 29) / 30, 128, s, d, srcBuf);
+            if (d.n <= 30 * d.sms)
+                launch_dependent(k_iter_small<R, 256, 1>, small, 256, s, d, srcBuf);
+            else if (d.n <= 30 * 3 * d.sms)
+                launch_dependent(k_iter_bal<R, 32, 128, 3>, small, 128, s, d, srcBuf);
             else
-                k_iter_bal<R, 128, 128, 3><<<(d.n + 125) / 126, 128, 0, s>>>(d, srcBuf);
+                k_iter_bal<R, 128, 128, 3><<<large, 128, 0, s>>>(d, srcBuf);
         }
     } else if (pipe) {
         if (lanes == 4) YB_ITER(256, 4, 2, true);

@@ -181,30 +181,52 @@ __device__ __forceinline__ void end_vertex(const Dev<R>& d, int i, int fb, int c
 }
 
 // ---------------------------------------------------------------------------------------
+// The costly parts of a vertex's own terms that need no sums: a kernel whose owning threads wait for
+// contacts forms them meanwhile.  Unconditional, and only the parts, so that the compiler fuses
+// the multiplies and adds of add_own_terms as it does without them.
+template <typename R>
+struct OwnParts {
+    Q<R> q0;     // orientation of segment k
+    R inertia;   // m / h^2 (used for free vertices)
+    R invl;      // 1 / lRest, and
+    V3<R> axis;  // the segment's direction by its orientation (used for segments)
+};
+
+template <typename R>
+__device__ __forceinline__ OwnParts<R> own_parts(const Dev<R>& d, int k, const V4<R>* __restrict__ QO,
+                                                 const SceneParams<R>& sp) {
+    OwnParts<R> w;
+    w.q0 = qof(QO[k]);
+    w.axis = qrotate(w.q0, V3<R>(R(1), R(0), R(0)));
+    w.invl = R(1) / d.vp[k].lRest;
+    w.inertia = R(1) / (d.pos[k].w * sp.hh);
+    return w;
+}
+
 // The vertex's own terms (cosserat.cu:40-81) added to force and Hessian sums that already hold
 // its contacts: inertia (H = m/h^2, f = m/h^2 (y - dx), y = h v + h^2 g formed here), the glue
 // spring to a connected vertex, and the stretch-shear coupling of segment k to its orientation
 // (its other endpoint's share in fb, Hb).  Also returns the vertex's flags, mass, segment
-// constants, step limit and orientation.
+// constants, step limit and orientation.  early: own_parts formed before, or null.
 template <typename R>
 __device__ __forceinline__ void add_own_terms(const Dev<R>& d, int k, const D2<R>* __restrict__ DX,
                                               const V4<R>* __restrict__ QO, const SceneParams<R>& sp, const V3<R>& p0,
                                               const V3<R>& e, const V3<R>& dx, const V3<R>& dx1, V3<R>& fa, H3<R>& Ha,
                                               V3<R>& fb, H3<R>& Hb, uint32_t& flags, R& invMass, R& lRest, R& kStretch,
-                                              R& sl, Q<R>& q0) {
+                                              R& sl, Q<R>& q0, const OwnParts<R>* early = nullptr) {
     const VP<R> vp = d.vp[k];
     flags = vp.flags;
     lRest = vp.lRest;
     kStretch = vp.kStretch;
     invMass = d.pos[k].w;
-    q0 = qof(QO[k]);
+    q0 = early ? early->q0 : qof(QO[k]);
     const R D = sp.D;
     if (invMass != R(0)) {
         const V4<R> v = d.vel[k];
         const R hh = sp.hh;
         const V3<R> y(sp.h * v.x + hh * sp.gx, sp.h * v.y + hh * sp.gy, sp.h * v.z + hh * sp.gz);
-        Ha.add_diag(R(1) / (invMass * hh));
-        fa += (R(1) / (hh * invMass)) * (y - dx);
+        Ha.add_diag(early ? early->inertia : R(1) / (invMass * hh));
+        fa += (early ? early->inertia : R(1) / (hh * invMass)) * (y - dx);
     }
     if (vp.cid >= 0) {
         const R stiff = R(40);
@@ -215,8 +237,8 @@ __device__ __forceinline__ void add_own_terms(const Dev<R>& d, int k, const D2<R
     }
     if (flags & F_HAS_NEXT) {
         sl = d.stepLim[k];
-        const R invl = R(1) / lRest;
-        const V3<R> c = (e + (dx1 - dx)) * invl - qrotate(q0, V3<R>(R(1), R(0), R(0)));
+        const R invl = early ? early->invl : R(1) / lRest;
+        const V3<R> c = (e + (dx1 - dx)) * invl - (early ? early->axis : qrotate(q0, V3<R>(R(1), R(0), R(0))));
         const R ks = kStretch * invl;
         R dd = ks * invl;
         fa += ks * c - (D * dd) * dx;
