@@ -64,7 +64,10 @@ struct alignas(sizeof(R) * 2) R2 {
     R x, y;
 };
 
-constexpr int RELCAP = 16;  // staged contacts: RELCAP x vertices slots in all (a contact past them is gathered)
+// Staged contacts: RELCAP x vertices slots in all; a contact past them is gathered and never certified
+// out of range (with 8 the Newton launches of a bundle with 13.7 contacts a segment take 370 us
+// instead of 171).  Simulations of more than an eighth of the free device memory have RELCAP_LARGE.
+constexpr int RELCAP = 16, RELCAP_LARGE = 7;
 constexpr int LIST_THREADS = 128;  // vertices per block of the list pass (one packed-offset tile)
 constexpr int SMALL_TILE = 32;     // ... in a small simulation
 __host__ __device__ constexpr int list_tiles(int n) { return (n + SMALL_TILE - 1) / SMALL_TILE; }  // at most

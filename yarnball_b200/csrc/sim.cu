@@ -11,9 +11,9 @@
 //   Sim::detectCollisions               sim/collision.cu:94-119
 //   Sim::printCollisionStats            sim/statistics.cpp:5-23
 //
-// One substep on the device is: predictor -> [detection: BVH rebuild or refit, traversal
-// (+ step limit)] or [step limit] -> numItr fused Newton/orientation iterations ->
-// advection.  No step reads anything back to the host (the reference's BVH query returns
+// One substep on the device is: predictor -> [detection: rebuild of the clusters (or BVH) or
+// their boxes, pair search, lists (+ step limit)] or [step limit] -> numItr fused
+// Newton/orientation iterations -> advection.  No step reads anything back to the host (the reference's BVH query returns
 // its pair count to the host every detection); each of the three substep shapes is captured
 // once as a CUDA graph and replayed.
 #include <algorithm>
@@ -327,6 +327,7 @@ struct Engine : EngineBase {
     }
 
     size_t allocBytes = 0;
+    size_t relSlots = RELCAP;  // staged contacts a vertex, on average
 
     yb_status alloc() {
         const size_t n = (size_t)S->capVerts;
@@ -349,6 +350,7 @@ struct Engine : EngineBase {
         want((void**)&d.stepLim, sizeof(R) * n);
         want((void**)&d.numCols, sizeof(int) * n);
         want((void**)&d.cols, sizeof(int) * n * MAX_COLS);
+        const size_t staged = req.size();  // these three: RELCAP slots a vertex, or fewer (below)
         want((void**)&d.relA, sizeof(V4<R>) * n * RELCAP);
         want((void**)&d.relB, sizeof(R2<R>) * n * RELCAP);
         want((void**)&d.relD, sizeof(R) * n * RELCAP);
@@ -402,8 +404,28 @@ struct Engine : EngineBase {
         want((void**)&rootBoxes, sizeof(float) * 6 * ns);
         want((void**)&diagPart, sizeof(double) * 8 * ((n + 255) / 256 + 1));
         want((void**)&sceneDelta, sizeof(int) * ns);
-        for (auto& r : req) off += (r.second + 255) & ~(size_t)255;
-        YB_CUDA(cudaMalloc(&block, off));
+        auto total = [&](size_t slots) {
+            size_t sum = 0;
+            for (size_t i = 0; i < req.size(); i++) {
+                if (i >= staged && i < staged + 3) req[i].second = req[i].second / relSlots * slots;
+                sum += (req[i].second + 255) & ~(size_t)255;
+            }
+            relSlots = slots;
+            return sum;
+        };
+        // A simulation that takes much of the device stages fewer contacts (the rest are gathered), and one
+        // that would not fit stages hardly any.
+        size_t freeBytes = 0, deviceBytes = 0;
+        YB_CUDA(cudaMemGetInfo(&freeBytes, &deviceBytes));
+        off = total(RELCAP);
+        if (off > freeBytes / 8) off = total(RELCAP_LARGE);
+        cudaError_t got = cudaMalloc(&block, off);
+        if (got == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            off = total(1);
+            got = cudaMalloc(&block, off);
+        }
+        YB_CUDA(got);
         allocBytes = off;
         off = 0;
         for (auto& r : req) {
@@ -415,7 +437,7 @@ struct Engine : EngineBase {
         d.nseg = 0;
         d.sp = spDev;
         d.csrCap = (unsigned)csrCap;
-        d.relCap = (unsigned)(n * RELCAP);
+        d.relCap = (unsigned)(n * relSlots);
         {
             int dev = 0, sms = 148;
             cudaGetDevice(&dev);
