@@ -159,7 +159,7 @@ yb_status yb_step(yb_sim* sim, float dt);
 /* Sim::stepCount, YarnBall.h:163. */
 yb_status yb_step_count(yb_sim* sim, uint64_t* out);
 
-/* Sim::bounds, YarnBall.cu:87-89: root box of the BVH (padded segment boxes) after the
+/* Sim::bounds, YarnBall.cu:87-89: root box of the broadphase (padded segment boxes) after the
  * last detection; minmax = {min x,y,z, max x,y,z}.  scene < 0 gives the union. */
 yb_status yb_bounds(yb_sim* sim, int32_t scene, float minmax[6]);
 
@@ -181,9 +181,9 @@ const char* yb_status_string(yb_status s);
 
 /* Engine tuning of the Newton kernel: threads per block, lanes per vertex (lanes split a
  * segment's contact loop; 0 selects a load-balanced kernel that flattens contact lists) and
- * software pipelining of the contact loop (with lanes 0: flatten per warp instead of per
- * block); valid shapes: (128, 0, 0|1), (128|256, 1, 0|1), (256, 2, 0), (256, 4, 0|1),
- * (512, 4, 0), (256|512, 8, 0).  useGraphs: replay captured CUDA graphs per substep.
+ * software pipelining of the contact loop (with lanes 0 it makes no difference); valid shapes:
+ * (128, 0, 0|1), (128|256, 1, 0|1), (256, 2, 0), (256, 4, 0|1), (512, 4, 0), (256|512, 8, 0).
+ * useGraphs: replay captured CUDA graphs per substep.
  * Default (128, 0, 0), the load-balanced kernel, graphs on. */
 yb_status yb_set_tuning(yb_sim* sim, int32_t iterThreads, int32_t lanesPerVertex, int32_t pipelined,
                         int32_t useGraphs);
@@ -204,8 +204,8 @@ yb_status yb_set_traversal(yb_sim* sim, int32_t packet);
 yb_status yb_get_traversal(yb_sim* sim, int32_t* packet);
 
 /* Simulations of at most 256 vertices advance all substeps of an advance() in one launch of a
- * one-block kernel (enable = 1, the default); enable = 0 uses the multi-block kernels and the
- * BVH.  Both run the same device functions in the same order (the load-balanced Newton
+ * one-block kernel (enable = 1, the default); enable = 0 uses the multi-block kernels.
+ * Both run the same device functions in the same order (the load-balanced Newton
  * kernel's summation order); they agree to rounding, since the compiler may fuse multiply-adds
  * differently inside the one kernel. */
 yb_status yb_set_small_path(yb_sim* sim, int32_t enable);
@@ -216,8 +216,8 @@ yb_status yb_set_stream(yb_sim* sim, void* stream);
 
 /* advance(dt) with every kernel class bracketed by CUDA events on the simulation's stream
  * (no graphs): msByClass[c] accumulates device milliseconds and launchesByClass[c] the
- * launches of class c: 0 predictor, 1 BVH rebuild (bounds, Morton, sort, Karras, refit),
- * 2 BVH refit, 3 traversal + step limit, 4 step limit alone, 5 Newton/orientation
+ * launches of class c: 0 predictor, 1 broadphase rebuild (keys, sort, boxes; with a
+ * BVH also its tree), 2 boxes alone (BVH refit), 3 pair search + step limit, 4 step limit alone, 5 Newton/orientation
  * iteration, 6 advection.  Arrays hold YB_PROFILE_CLASSES entries. */
 #define YB_PROFILE_CLASSES 7
 yb_status yb_profile_advance(yb_sim* sim, float dt, double* msByClass, uint64_t* launchesByClass);

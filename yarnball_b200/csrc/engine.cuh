@@ -47,6 +47,8 @@ enum {
     EW_MAX_COLS = 4,     // largest contact count of any segment (cumulative max)
     EW_MIN_DIST = 5,     // float bits of the smallest centre-line distance of any listed contact
                          // at substep start (cumulative min; +inf before the first contact)
+    EW_IN_RANGE = 6,     // of the contacts in a sample of the list passes' tiles: those in the barrier's
+    EW_LISTED = 7,       // range at substep start, and all (both cumulative, modulo 2^32)
     EW_COUNT = 8
 };
 enum { IE_BVH_STACK = 1, IE_SORT_WAIT = 2, IE_GRID_WAIT = 4, IE_REFIT = 8, IE_LIST_WAIT = 16, IE_CONTACT = 32 };
@@ -203,6 +205,7 @@ struct Dev {
     int* sceneRoot;   // child code of each scene's subtree root (or INT_MIN when empty)
     int* sceneLast;   // sorted position of the last leaf of each scene's subtree
     unsigned* travNext;   // next query (sorted position) handed out by the traversal
+    int sift;             // 0: k_iter_all where newton_may_take_all, else the kernels that test contacts first
     int travBlocks[2];    // persistent traversal grid of the BVH walks (travPacket 0, 1)
     int travPacket;       // 2: cluster pairs (k_pairs, default), 1: one BVH walk per warp for 32
                           // queries (k_traverse_packet), 0: one per lane (k_traverse)
@@ -248,6 +251,12 @@ void launch_dependent(void (*kernel)(P...), size_t blocks, unsigned threads, cud
 // Hint: bring the line holding p into L1 (no register is held until the data is used).
 __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+// Sizes at which k_iter_all can be the better Newton kernel: more than one wave of its blocks.
+template <typename R>
+bool newton_may_take_all(const Dev<R>& d) {
+    return sizeof(R) == 4 && d.n > 126 * 7 * d.sms;
 }
 
 // --- kernel launchers (stream-ordered; no host synchronisation) ---

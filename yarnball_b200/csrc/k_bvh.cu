@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     }
     R m = R(0);
     if (valid) m = step_limit_base(d, k, d.sp[sc]);
-    int pens = 0;
+    int pens = 0, near = 0;
     float dmin = INFINITY;
     for (int b0 = 0; b0 < total; b0 += NT) {
         const int f = b0 + t;
@@ -774,6 +774,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
             lim = contact_step_limit(d, ks, g < (unsigned long long)d.relCap ? (size_t)g : NO_STAGE, o, oa0, oa1,
                                      d.sp[sScene[s]], pen, dist);
             pens += pen;
+            near += dist <= d.sp[sScene[s]].outOfRange;
             dmin = fminf(dmin, (float)dist);
         }
         sLim[t] = lim;
@@ -785,6 +786,11 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     if (pens) {
         atomicAdd(&d.err[EW_PENETRATIONS], pens);
         d.err[EW_WARNING] = 2;
+    }
+    if (tile % 16 == 0) {  // a sample of the contacts, for the choice of the Newton kernel
+        near = __reduce_add_sync(0xffffffffu, near);
+        if ((t & 31) == 0 && near) atomicAdd(&d.err[EW_IN_RANGE], near);
+        if (t == 0 && total) atomicAdd(&d.err[EW_LISTED], total);
     }
     // distances are >= 0, whose float bit patterns order like the integers
 #pragma unroll

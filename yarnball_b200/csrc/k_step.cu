@@ -536,6 +536,230 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
 }
 
 // ---------------------------------------------------------------------------------------
+// The same iteration without the test: every contact is evaluated, NT at a time, one per thread.
+// The better one for large simulations whose listed contacts are mostly in range (settled piles):
+// there the test costs more than the few contacts it spares.  72 registers, 7 blocks an SM.  Bound by
+// issue and the latency of the gathers.  Measured, us a launch, k_iter_bal against this kernel by the
+// share of listed contacts that are in range when a substep starts: 1.0M vertices in 32 scenes, 17 %:
+// 100 against 119, 32 %: 119 / 128, 46 %: 142 / 140, 53 %: 164 / 156, 57 %: 180 / 169; 8.4M in 269 scenes,
+// 34 %: 943 / 986, 47 %: 1080 / 1047, 55 %: 1207 / 1134; pile of 262,144 vertices, 48 %: 108 / 111, 57 %:
+// 107 / 101, 61 %: 104 / 93; pile of 65,792, where the grid is less than a wave, 58 %: 35 / 37.
+// Results are the same bit for bit.
+template <typename R, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
+    after_previous_kernel();
+    constexpr int B = NT;
+    constexpr int CORE = B - 2;
+    constexpr int NW = NT / 32;
+    const int t = threadIdx.x;
+    const int k = blockIdx.x * CORE - 1 + t;
+    const int n = d.n;
+    const bool valid = (k >= 0) && (k < n);
+    const D2<R>* __restrict__ DX = d.dx[src];
+    const V4<R>* __restrict__ QO = d.q[src];
+
+    __shared__ R sSeg[12][B];  // p0, e = p1 - p0, dx, dx1 of each slot's segment
+    // contributions of one chunk of contacts, double buffered, in 16-byte groups:
+    // (fa, fb.x) (fb.yz, Ha0-1) (Ha2-5) (Hb0-3), then (Hb4-5)
+    __shared__ V4<R> sCon4[2][4][B];
+    __shared__ R2<R> sCon2[2][B];
+    __shared__ int sOwn[2][B];     // owning slot of each contact of a chunk (double buffered)
+    __shared__ int sOff[B + 1];
+    __shared__ int sScene[B];
+    __shared__ int sWarp[NW];
+    __shared__ unsigned sBase;
+
+    // The contact loop runs first and accumulates from zero; the vertex's own terms (inertia,
+    // glue, stretch) are loaded and added after it, so their inputs are not live (in
+    // registers) across the loop.
+    V3<R> fa(R(0)), fb(R(0));
+    H3<R> Ha, Hb;
+    Ha.zero(); Hb.zero();
+    int nc = 0, sc = 0;
+    if (t == 0) sBase = d.csrOff[k < 0 ? 0 : k];  // the block's first packed slot (k < n here)
+    {
+        V3<R> p0(R(0)), e(R(0)), dx(R(0)), dx1(R(0));
+        if (valid) {
+            // inputs of the vertex's own terms, used after the contact loop
+            prefetch_l1(d.vel + k);
+            prefetch_l1(QO + k);
+            prefetch_l1(d.qRest + k);
+            prefetch_l1(d.stepLim + k);
+            const uint32_t fl = d.vp[k].flags;
+            sc = scene_of(fl);
+            const D2<R> own = DX[k];
+            dx = xyz(own.a);
+            dx1 = xyz(own.b);
+            p0 = xyz(d.pos[k]);
+            if (fl & F_HAS_NEXT) {
+                e = xyz(d.pos[k + 1]) - p0;
+                unsigned off;
+                nc = contact_range(d, k, off);
+            }
+        }
+        sSeg[0][t] = p0.x; sSeg[1][t] = p0.y; sSeg[2][t] = p0.z;
+        sSeg[3][t] = e.x; sSeg[4][t] = e.y; sSeg[5][t] = e.z;
+        sSeg[6][t] = dx.x; sSeg[7][t] = dx.y; sSeg[8][t] = dx.z;
+        sSeg[9][t] = dx1.x; sSeg[10][t] = dx1.y; sSeg[11][t] = dx1.z;
+        sScene[t] = sc;
+    }
+    // block exclusive scan of the contact counts (the block's packed slots are base + offset)
+    {
+        const int lane = t & 31, w = t >> 5;
+        int x = nc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) sWarp[w] = x;
+        __syncthreads();
+        int wo = 0;
+        for (int i = 0; i < w; i++) wo += sWarp[i];
+        sOff[t] = wo + x - nc;
+        if (t == B - 1) sOff[B] = wo + x;
+        __syncthreads();
+    }
+    int total = sOff[B];
+    int myOff = sOff[t];
+    const unsigned base = sBase;
+    if (base > d.csrCap || d.csrCap - base < (unsigned)total) {  // only a packing the list pass reported as failed
+        total = 0;
+        myOff = 0;
+        nc = 0;
+    }
+    // Chunks of NT contacts, one per thread.  Each thread writes its own slot index over its
+    // contacts of the next chunk before the current chunk's barrier, which publishes it, and
+    // the contributions are double buffered: a buffer is written again only after the next
+    // chunk's barrier, which every thread reaches after summing it, so each chunk needs one
+    // barrier.
+    for (int g = myOff; g < min(myOff + nc, NT); g++) sOwn[0][g] = t;
+    __syncthreads();
+    int buf = 0;
+    // The partner id of this thread's contact is loaded one chunk ahead (after the previous
+    // chunk's barrier, before its summation), so a chunk starts with the partner gather.
+    int jn = 0;
+    if (t < total) jn = __ldg(d.csrCols + (base + t));
+    for (int b0 = 0; b0 < total; b0 += NT, buf ^= 1) {
+        const int f = b0 + t;
+        {
+            const int nb = b0 + NT;
+            const int g1 = min(myOff + nc, nb + NT);
+            for (int g = max(myOff, nb); g < g1; g++) sOwn[buf ^ 1][g - nb] = t;
+        }
+        V3<R> cfa(R(0)), cfb(R(0));
+        H3<R> cHa, cHb;
+        cHa.zero(); cHb.zero();
+        if (f < total && partner_ok(d, jn)) {
+            const int s = sOwn[buf][t];
+            const int j = jn;
+            const V3<R> sp0(sSeg[0][s], sSeg[1][s], sSeg[2][s]);
+            V3<R> r0, r1;
+            partner_rel(d, base + f, j, sp0, r0, r1);
+            const D2<R> pd = DX[j];
+            const V3<R> se(sSeg[3][s], sSeg[4][s], sSeg[5][s]);
+            const V3<R> sdx(sSeg[6][s], sSeg[7][s], sSeg[8][s]);
+            const V3<R> sdx1(sSeg[9][s], sSeg[10][s], sSeg[11][s]);
+            contact_term(se, sdx, sdx1, r0, r1, xyz(pd.a), xyz(pd.b), d.sp[sScene[s]], cfa, cHa, cfb, cHb);
+        }
+        {
+            V4<R> w;
+            w.x = cfa.x; w.y = cfa.y; w.z = cfa.z; w.w = cfb.x; sCon4[buf][0][t] = w;
+            w.x = cfb.y; w.y = cfb.z; w.z = cHa.d[0]; w.w = cHa.d[1]; sCon4[buf][1][t] = w;
+            w.x = cHa.d[2]; w.y = cHa.d[3]; w.z = cHa.d[4]; w.w = cHa.d[5]; sCon4[buf][2][t] = w;
+            w.x = cHb.d[0]; w.y = cHb.d[1]; w.z = cHb.d[2]; w.w = cHb.d[3]; sCon4[buf][3][t] = w;
+            R2<R> w2;
+            w2.x = cHb.d[4]; w2.y = cHb.d[5];
+            sCon2[buf][t] = w2;
+        }
+        __syncthreads();
+        {
+            // next chunk: partner id, and the staged partner positions into L1
+            const int fn = b0 + NT + t;
+            if (fn < total) {
+                const unsigned g = base + fn;
+                jn = __ldg(d.csrCols + g);
+                if (g < d.relCap) {
+                    prefetch_l1(d.relA + g);
+                    prefetch_l1(d.relB + g);
+                }
+            }
+        }
+        const int f0 = max(myOff, b0), f1 = min(myOff + nc, b0 + NT);
+        for (int g = f0; g < f1; g++) {
+            const int i = g - b0;
+            const V4<R> w0 = sCon4[buf][0][i], w1 = sCon4[buf][1][i], w2 = sCon4[buf][2][i], w3 = sCon4[buf][3][i];
+            const R2<R> w4 = sCon2[buf][i];
+            fa += V3<R>(w0.x, w0.y, w0.z);
+            fb += V3<R>(w0.w, w1.x, w1.y);
+            Ha.d[0] += w1.z; Ha.d[1] += w1.w;
+            Ha.d[2] += w2.x; Ha.d[3] += w2.y; Ha.d[4] += w2.z; Ha.d[5] += w2.w;
+            Hb.d[0] += w3.x; Hb.d[1] += w3.y; Hb.d[2] += w3.z; Hb.d[3] += w3.w;
+            Hb.d[4] += w4.x; Hb.d[5] += w4.y;
+        }
+    }
+
+    // The halo exchange after the loop uses the contribution buffer the last chunk did not
+    // use (buf), viewed as 16 rows of B values: every thread finished reading it before the
+    // last chunk's barrier.
+    R (*rows)[B] = reinterpret_cast<R (*)[B]>(&sCon4[buf][0][0]);
+    R (*sFb)[B] = rows;       // rows 0-2
+    R (*sHb)[B] = rows + 3;   // rows 3-8
+    R* sSL = rows[9];
+    R (*sDX)[B] = rows + 10;  // rows 10-12
+
+    // the vertex's own terms (cosserat.cu:40-81)
+    R sl = yinf<R>();
+    uint32_t flags = 0;
+    R invMass = R(0), lRest = R(1), kStretch = R(0);
+    const V3<R> p0(sSeg[0][t], sSeg[1][t], sSeg[2][t]);
+    const V3<R> e(sSeg[3][t], sSeg[4][t], sSeg[5][t]);
+    const V3<R> dx(sSeg[6][t], sSeg[7][t], sSeg[8][t]);
+    Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
+    const SceneParams<R>* spp = d.sp;
+    if (valid) {
+        spp = &d.sp[sc];
+        add_own_terms(d, k, DX, QO, *spp, p0, e, dx, V3<R>(sSeg[9][t], sSeg[10][t], sSeg[11][t]), fa, Ha, fb, Hb,
+                      flags, invMass, lRest, kStretch, sl, q0);
+    }
+
+    sFb[0][t] = fb.x; sFb[1][t] = fb.y; sFb[2][t] = fb.z;
+#pragma unroll
+    for (int q = 0; q < 6; q++) sHb[q][t] = Hb.d[q];
+    sSL[t] = sl;
+    __syncthreads();
+
+    V3<R> dxn = dx;
+    if (valid && t > 0) {
+        if (flags & F_HAS_PREV) {
+            fa += V3<R>(sFb[0][t - 1], sFb[1][t - 1], sFb[2][t - 1]);
+            H3<R> hp;
+#pragma unroll
+            for (int q = 0; q < 6; q++) hp.d[q] = sHb[q][t - 1];
+            Ha.add(hp);
+            sl = ymin(sl, sSL[t - 1]);
+        }
+        if (invMass != R(0)) {
+            dxn = dx + spp->accel * solve3(Ha, fa);
+            const R l = len(dxn);
+            if (l > sl && l > R(0)) dxn *= sl / l;
+        }
+    }
+    sDX[0][t] = dxn.x; sDX[1][t] = dxn.y; sDX[2][t] = dxn.z;
+    const bool core = valid && t >= 1 && t <= CORE;
+    __syncthreads();
+
+    if (core) {
+        const V3<R> dxb(sDX[0][t + 1], sDX[1][t + 1], sDX[2][t + 1]);
+        D2<R> o;
+        o.a = v4(dxn, R(0));
+        o.b = v4(k + 1 < n ? dxb : V3<R>(R(0)), R(0));
+        d.dx[src ^ 1][k] = o;
+        d.q[src ^ 1][k] = v4of(orientation_update(d, k, QO, flags, e, dxn, dxb, lRest, kStretch, q0));
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // The same iteration for small simulations, where a launch lasts as long as one block's chain of
 // dependent steps (some 10k cycles) and most of the chip's issue slots are free.  A block has 32
 // slots: warp 0 owns them, the other warps work on the contacts in the same two stages.  While they
@@ -828,6 +1052,8 @@ void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, 
                 launch_dependent(k_iter_bal<R, 32, 256, 3>, small, 256, s, d, srcBuf);
             else if (d.n <= 30 * 6 * d.sms)
                 launch_dependent(k_iter_bal<R, 32, 128, 6>, small, 128, s, d, srcBuf);
+            else if (!d.sift && newton_may_take_all(d))
+                launch_dependent(k_iter_all<R, 128, 7>, large, 128, s, d, srcBuf);
             else if (d.n <= 126 * 6 * d.sms)
                 k_iter_bal<R, 128, 128, 6><<<large, 128, 0, s>>>(d, srcBuf);
             else

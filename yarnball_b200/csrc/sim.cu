@@ -310,7 +310,8 @@ struct Engine : EngineBase {
     int* errHost = nullptr;
     cudaGraphExec_t graphs[GRAPH_TYPES] = {nullptr, nullptr, nullptr};
     uint64_t graphLaunches[GRAPH_TYPES] = {0, 0, 0};
-    int graphItr = -1, graphThreads = -1, graphLanes = -1, graphPipe = -1, graphNseg = -1;
+    int graphItr = -1, graphThreads = -1, graphLanes = -1, graphPipe = -1, graphNseg = -1, graphSift = -1;
+    unsigned listedSeen = 0, inRangeSeen = 0;  // the sampled contact counts at the last check
     int keyBits = CURVE_BITS;
     int64_t penTotal = 0;
     float minDist = INFINITY;
@@ -446,6 +447,7 @@ struct Engine : EngineBase {
             d.sms = sms;
         }
         d.travPacket = S->travPacket;
+        d.sift = 1;
         YB_CUDA(small_path_prepare<R>());  // a recycled batch may become small later
         YB_CUDA(cudaHostAlloc((void**)&spHost, sizeof(SceneParams<R>) * ns, cudaHostAllocDefault));
         YB_CUDA(cudaHostAlloc((void**)&errHost, sizeof(int) * EW_COUNT, cudaHostAllocDefault));
@@ -874,7 +876,7 @@ struct Engine : EngineBase {
             if (g) cudaGraphExecDestroy(g);
             g = nullptr;
         }
-        graphItr = graphThreads = graphLanes = graphPipe = graphNseg = -1;
+        graphItr = graphThreads = graphLanes = graphPipe = graphNseg = graphSift = -1;
     }
 
     yb_status run_substep(int type) override {
@@ -885,13 +887,14 @@ struct Engine : EngineBase {
             return YB_OK;
         }
         if (graphItr != num_itr() || graphThreads != S->iterThreads || graphLanes != S->iterLanes ||
-            graphPipe != S->iterPipe || graphNseg != d.nseg) {
+            graphPipe != S->iterPipe || graphNseg != d.nseg || graphSift != d.sift) {
             invalidate_graphs();
             graphItr = num_itr();
             graphThreads = S->iterThreads;
             graphLanes = S->iterLanes;
             graphPipe = S->iterPipe;
             graphNseg = d.nseg;
+            graphSift = d.sift;
         }
         if (!graphs[type]) {
             cudaGraph_t g = nullptr;
@@ -913,6 +916,21 @@ struct Engine : EngineBase {
     }
 
     // atHost: the kernel before wrote the error words to host memory itself.
+    // The Newton kernel of the following substeps, by the share of the sampled contacts that were in
+    // range since the last check: above about a half, testing them first costs more than it spares (figures at
+    // k_iter_all).  Between the two bounds the choice stays, so that graphs are seldom captured anew.
+    // The results do not depend on it.
+    void choose_newton() {
+        const unsigned listed = (unsigned)errHost[EW_LISTED] - listedSeen;
+        const unsigned inRange = (unsigned)errHost[EW_IN_RANGE] - inRangeSeen;
+        listedSeen = (unsigned)errHost[EW_LISTED];
+        inRangeSeen = (unsigned)errHost[EW_IN_RANGE];
+        if (listed == 0 || inRange > listed || S->iterLanes != 0 || !newton_may_take_all(d)) return;
+        const double share = (double)inRange / listed;
+        if (share > 0.52) d.sift = 0;
+        if (share < 0.47) d.sift = 1;
+    }
+
     yb_status check_errors(bool atHost = false) override {
         YB_CUDA(cudaGetLastError());
         if (!atHost)
@@ -920,6 +938,7 @@ struct Engine : EngineBase {
         YB_CUDA(cudaStreamSynchronize(S->stream));
         yb_status st = YB_OK;
         penTotal = errHost[EW_PENETRATIONS];
+        choose_newton();
         std::memcpy(&minDist, &errHost[EW_MIN_DIST], sizeof(float));
         if (errHost[EW_ERROR] != 0) {
             S->lastErrorCode = errHost[EW_ERROR];
