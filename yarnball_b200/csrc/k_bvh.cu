@@ -524,16 +524,29 @@ __global__ void __launch_bounds__(TRAV_THREADS) k_traverse(Dev<R> d) {
 // 16 entries is sorted by its own thread with a bitonic network on 16 registers; a longer one
 // by the whole warp, one list at a time, as a bitonic sort of 128 entries held four per lane
 // (entry i = 32 r + lane): steps with a stride of 32 or more swap within a lane, smaller ones
-// exchange between lanes.  Padding entries are INT_MAX and sort to the end.
+// exchange between lanes.  Padding entries are INT_MAX and sort to the end.  The sorted lists are
+// also left in shared memory, each from its place `off` on, as far as `room` entries go, with the
+// thread that owns them.
+// A thread reads and writes its row (512 bytes, so 16-byte aligned) 4 entries at a time: every access of
+// a warp touches 32 lines, and the kernel is bound by these.
 template <typename R>
-__device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
+__device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n, int off, int room, int* ids,
+                                          unsigned char* owner) {
     constexpr int PAD = 0x7fffffff;
+    static_assert(MAX_COLS % 4 == 0, "rows are read by 4 entries");
     const int lane = threadIdx.x & 31;
-    if (k >= 0 && n > 1 && n <= 16) {
-        int* __restrict__ cl = d.cols + col_at(k, 0);
+    if (k >= 0 && n >= 1 && n <= 16) {
+        int4* __restrict__ row = reinterpret_cast<int4*>(d.cols + col_at(k, 0));
         int v[16];
 #pragma unroll
-        for (int a = 0; a < 16; a++) v[a] = a < n ? cl[a] : PAD;
+        for (int a = 0; a < 16; a += 4) {
+            int4 w = make_int4(PAD, PAD, PAD, PAD);
+            if (a < n) w = row[a / 4];
+            v[a] = w.x;
+            v[a + 1] = a + 1 < n ? w.y : PAD;
+            v[a + 2] = a + 2 < n ? w.z : PAD;
+            v[a + 3] = a + 3 < n ? w.w : PAD;
+        }
 #pragma unroll
         for (int sz = 2; sz <= 16; sz <<= 1) {
 #pragma unroll
@@ -552,8 +565,14 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
             }
         }
 #pragma unroll
+        for (int a = 0; a < 16; a += 4)
+            if (a < n) row[a / 4] = make_int4(v[a], v[a + 1], v[a + 2], v[a + 3]);
+#pragma unroll
         for (int a = 0; a < 16; a++)
-            if (a < n) cl[a] = v[a];
+            if (a < n && off + a < room) {
+                ids[off + a] = v[a];
+                owner[off + a] = (unsigned char)threadIdx.x;
+            }
     }
     unsigned longLists = __ballot_sync(0xffffffffu, k >= 0 && n > 16);
     while (longLists) {
@@ -561,6 +580,7 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
         longLists &= longLists - 1;
         const int kk = __shfl_sync(0xffffffffu, k, src);
         const int m = __shfl_sync(0xffffffffu, n, src);
+        const int at = __shfl_sync(0xffffffffu, off, src);
         int* __restrict__ cl = d.cols + col_at(kk, 0);
         int v[4];
 #pragma unroll
@@ -600,7 +620,13 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n) {
 #pragma unroll
         for (int r = 0; r < 4; r++) {
             const int i = 32 * r + lane;
-            if (i < m) cl[i] = v[r];
+            if (i < m) {
+                cl[i] = v[r];
+                if (at + i < room) {
+                    ids[at + i] = v[r];
+                    owner[at + i] = (unsigned char)((threadIdx.x & ~31u) + src);
+                }
+            }
         }
         __syncwarp();
     }
@@ -633,6 +659,10 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     __shared__ R sA0[3][B], sA1[3][B];
     __shared__ int sScene[B];
     __shared__ R sLim[NT];
+    constexpr int HELD = B == 128 ? 8 * B : 16 * B;  // sorted contacts kept here for the second half
+    __shared__ int sId[HELD];
+    __shared__ unsigned char sOwner[HELD];
+    static_assert(B <= 256, "owners are bytes");
     after_previous_kernel();
     const int t = threadIdx.x;
     const bool owns = B == NT || t < B;  // the others only help with the contacts
@@ -686,7 +716,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
         if ((t & 31) == 0 && m) atomicMax(&d.err[EW_MAX_COLS], m);
-        sort_list(d, valid ? k : -1, nc);
+        sort_list(d, valid ? k : -1, nc, sOff[t], HELD, sId, sOwner);
     }
     if (owns) {
         sScene[t] = sc;
@@ -754,14 +784,20 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
         const int f = b0 + t;
         R lim = yinf<R>();
         if (f < total) {
-            int lo = 0, hi = B - 1;  // owner: the last slot whose offset is <= f
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (sOff[mid] <= f) lo = mid; else hi = mid - 1;
+            int slot, o;
+            if (sortLists && f < HELD) {
+                slot = sOwner[f];
+                o = sId[f];
+            } else {
+                int lo = 0, hi = B - 1;  // owner: the last slot whose offset is <= f
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (sOff[mid] <= f) lo = mid; else hi = mid - 1;
+                }
+                slot = lo;
+                o = d.cols[col_at(tile * B + slot, f - sOff[slot])];
             }
-            const int s = lo, c = f - sOff[s];
-            const int ks = tile * B + s;
-            const int o = d.cols[col_at(ks, c)];
+            const int s = slot, ks = tile * B + s;
             const unsigned long long g = base + (unsigned long long)f;
             if (g < (unsigned long long)d.csrCap) {
                 d.csrCols[g] = o;
