@@ -161,4 +161,13 @@ __device__ __forceinline__ R contact_step_limit(const Dev<R>& d, int k, size_t s
     return E::mul(safe, l);
 }
 
+// Minimum of step limits in shared memory: they are >= 0, so their bits order like them (and those of
+// something that is not a number are larger than infinity's: it is passed over, as in ymin).
+__device__ __forceinline__ void limit_min(float* at, float v) {
+    atomicMin(reinterpret_cast<unsigned*>(at), __float_as_uint(v));
+}
+__device__ __forceinline__ void limit_min(double* at, double v) {
+    atomicMin(reinterpret_cast<unsigned long long*>(at), (unsigned long long)__double_as_longlong(v));
+}
+
 }  // namespace yb

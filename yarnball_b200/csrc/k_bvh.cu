@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     __shared__ unsigned long long sBase;
     __shared__ R sA0[3][B], sA1[3][B];
     __shared__ int sScene[B];
-    __shared__ R sLim[NT];
+    __shared__ R sLim[B];  // each owner's smallest limit
     constexpr int HELD = B == 128 ? 8 * B : 16 * B;  // sorted contacts kept here for the second half
     __shared__ int sId[HELD];
     __shared__ unsigned char sOwner[HELD];
@@ -720,6 +720,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     }
     if (owns) {
         sScene[t] = sc;
+        sLim[t] = yinf<R>();
         sA0[0][t] = a0.x; sA0[1][t] = a0.y; sA0[2][t] = a0.z;
         sA1[0][t] = a1.x; sA1[1][t] = a1.y; sA1[2][t] = a1.z;
     }
@@ -782,7 +783,6 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
     float dmin = INFINITY;
     for (int b0 = 0; b0 < total; b0 += NT) {
         const int f = b0 + t;
-        R lim = yinf<R>();
         if (f < total) {
             int slot, o;
             if (sortLists && f < HELD) {
@@ -807,18 +807,16 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
             const V3<R> oa1(sA1[0][s], sA1[1][s], sA1[2][s]);
             bool pen = false;
             R dist;
-            lim = contact_step_limit(d, ks, g < (unsigned long long)d.relCap ? (size_t)g : NO_STAGE, o, oa0, oa1,
-                                     d.sp[sScene[s]], pen, dist);
+            const R lim = contact_step_limit(d, ks, g < (unsigned long long)d.relCap ? (size_t)g : NO_STAGE, o, oa0, oa1,
+                                             d.sp[sScene[s]], pen, dist);
+            limit_min(&sLim[s], lim);
             pens += pen;
             near += dist <= d.sp[sScene[s]].outOfRange;
             dmin = fminf(dmin, (float)dist);
         }
-        sLim[t] = lim;
-        __syncthreads();
-        const int f0 = max(myOff, b0), f1 = min(myOff + nc, b0 + NT);
-        for (int g = f0; g < f1; g++) m = ymin(m, sLim[g - b0]);
-        __syncthreads();
     }
+    __syncthreads();
+    if (owns) m = ymin(m, sLim[t]);
     if (pens) {
         atomicAdd(&d.err[EW_PENETRATIONS], pens);
         d.err[EW_WARNING] = 2;

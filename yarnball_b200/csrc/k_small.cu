@@ -60,13 +60,6 @@ struct SmallShare {
     SceneParams<R> sp[SMALL_SCENES];
 };
 
-__device__ __forceinline__ void small_min(float* at, float v) {
-    atomicMin(reinterpret_cast<unsigned*>(at), __float_as_uint(v));
-}
-__device__ __forceinline__ void small_min(double* at, double v) {
-    atomicMin(reinterpret_cast<unsigned long long*>(at), (unsigned long long)__double_as_longlong(v));
-}
-
 template <typename R>
 __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
     k_small(const __grid_constant__ Dev<R> g, const SceneParams<R>* params, int* errOut, int steps, int numItr,
@@ -253,7 +246,7 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                                              d.sp[scene_of(m.vp[a].flags)], pen, dist);
             pens += pen;
             dmin = fminf(dmin, (float)dist);
-            small_min(&m.stepLim[a], lim);  // limits are >= 0: their bits order like them
+            limit_min(&m.stepLim[a], lim);
         }
         __syncthreads();
         if (valid && !(seg && d.sp[sc].useStepLimit)) m.stepLim[k] = yinf<R>();
