@@ -642,9 +642,13 @@ __device__ __forceinline__ void sort_list(const Dev<R>& d, int k, int n, int off
 // IE_LIST_WAIT).  The tile's
 // contacts are then evaluated NT at a time, one per thread: the packed partner id, the
 // partner endpoints staged relative to p0 in the same slot, and the step-size limit
-// (collision.cu:121-159), of which each segment takes the minimum over its contacts in list
-// order (the minimum is exact, so this equals a per-segment loop).  The packed slots are
-// contiguous per tile, so the Newton iteration reads them coalesced.
+// (collision.cu:121-159), of which each segment takes the minimum over its contacts in shared
+// memory (the minimum is exact in any order, so this equals a per-segment loop).  The packed
+// slots are contiguous per tile, so the Newton iteration reads them coalesced.
+// Bound by latency (partner gathers) and issue (47 % of the slots).  Measured with the pair search, per
+// substep, entries one by one and minima by owners between barriers -> rows by 4 entries, ids and
+// owners in shared memory -> minima in shared memory: 8.4M vertices 3.32 -> 3.20 -> 3.13 ms, 1.0M
+// 403 -> 389 -> 376 us, pile of 262,144 302 -> 286 -> 274 us.
 constexpr int LIST_SPIN_LIMIT = 1 << 22;
 constexpr unsigned long long LS_AGG = 1ull << 62;
 constexpr unsigned long long LS_PRE = 2ull << 62;
@@ -1015,8 +1019,9 @@ void launch_lists(const Dev<R>& d, int sortLists, cudaStream_t s) {
     // A tile's contacts are worked NT at a time between barriers.  While the chip is far from full a
     // launch lasts as long as one tile's chain of steps, so small tiles get helper threads: the class
     // of the pair search and this pass takes 28 -> 23 us at 1,949 vertices, 54 -> 46 us in the FP64
-    // build at 12,827, 145 -> 134 us and 232 -> 218 us at 65,792 and 100,352, but 335 -> 349 us at
-    // 262,144 and 450 -> 554 us at 1.0M (a tile's fixed steps outweigh its contacts).
+    // build at 12,827, 145 -> 134 us and 232 -> 218 us at 65,792 and 100,352, but 274 -> 293 us at
+    // 262,144 and 450 -> 554 us at 1.0M (a tile's fixed steps outweigh its contacts).  256 threads for
+    // a tile of 128: 376 -> 413 us at 1.0M.
     const int tiles = (d.n + SMALL_TILE - 1) / SMALL_TILE;
     if (tiles <= 24 * d.sms)
         launch_dependent(k_lists<R, SMALL_TILE, 128>, tiles, 128, s, d, sortLists);
