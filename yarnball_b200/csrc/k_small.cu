@@ -22,7 +22,8 @@
 //     upwards gives the list in partner order without a sort.
 // Measured (B200, us per substep, before -> now, where before one thread ran each vertex with
 // all of its pairs and contacts in global memory): README scene (64 vertices, few contacts)
-// 53 -> 16; swatch of 216 vertices (2 contacts a segment) 209 -> 46.
+// 53 -> 15; swatch of 216 vertices (2 contacts a segment) 209 -> 46.  Testing contacts for being out of
+// range first, as k_iter_bal does: 46 -> 45, but 15 -> 16 in the README scene.
 //
 // Reference semantics: Sim::advance (sim/step.cpp:36-55) with initItr / endItr
 // (sim/iteration.cu), detectCollisions + buildCollisionList (sim/collision.cu:39-119),
