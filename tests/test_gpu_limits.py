@@ -1,0 +1,82 @@
+"""Inputs at the limits of what the engine accepts.
+
+Unbounded boxes: a predicted displacement whose square overflows single precision gives a segment
+a box without bounds and an infinite filter distance, so it is listed with every segment of its
+scene that is no neighbour of it, and with nothing else: not with the vertices that start no
+segment, and not with the places past a scene's last segment in a cluster of 32.  The lists of all
+broadphase paths are the same.
+"""
+import numpy as np
+import pytest
+
+from yarnball_b200 import scenes
+from yarnball_b200.sim import Sim
+
+pytestmark = pytest.mark.gpu
+
+H = 1e-3
+
+
+def _straight_yarns(counts, fast):
+    """Scenes of parallel yarns (`counts`: their lengths, scene by scene), far apart but for one
+    crossing pair; vertex `fast` of each scene moves by 1e20 in a substep."""
+    sizes = [sum(c) for c in counts]
+    sim = Sim(scenes=sizes)
+    off = 0
+    for lens in counts:
+        m = sum(lens)
+        x = np.zeros((m, 3), np.float32)
+        at = 0
+        for y, length in enumerate(lens):
+            x[at:at + length, 0] = np.arange(length) * 2e-3
+            x[at:at + length, 1] = (0.9e-3 if y == 1 else 0.02 * y)
+            at += length
+        scenes.fill_yarns(sim, x, np.asarray(lens, np.int32), offset=off, pin_first=True)
+        off += m
+    sim.set_meta_all(**scenes.PILE_META)
+    sim.configure()
+    sim.maxH = H
+    for o in sim.sceneOffsets[:-1]:
+        sim.vels[o + fast] = (1e23, -1e23, 1e23)
+    sim.upload()
+    return sim
+
+
+def _lists(sim):
+    nc, lists, _ = sim.debug_contacts()
+    return nc, lists
+
+
+UNBOUNDED = {
+    "one scene": [[13, 7]],
+    "a cluster and a part": [[20, 20]],
+    "two scenes": [[15, 6], [21, 9, 3]],
+    "whole warps": [[16, 16]],
+}
+
+
+@pytest.mark.parametrize("name", list(UNBOUNDED))
+@pytest.mark.parametrize("fast", [0, 4])
+def test_unbounded_boxes_meet_segments_only(name, fast):
+    counts = UNBOUNDED[name]
+    got = []
+    for mode in ("walk", "packets", "clusters", "one block"):
+        sim = _straight_yarns(counts, fast)
+        if mode == "one block":
+            sim.advance(H)  # one substep; the lists are those of its detection
+        else:
+            sim.set_small_path(False)
+            sim.set_traversal({"walk": 0, "packets": 1, "clusters": 2}[mode])
+            sim.debug_phases(1 | 2, H)
+        got.append(_lists(sim))
+        offs, segs = sim.sceneOffsets, (sim.verts["flags"] & 2) != 0
+        sim.close()
+    nc, lists = got[0]
+    for s in range(len(counts)):
+        here = np.nonzero(segs[offs[s]:offs[s + 1]])[0] + offs[s]
+        for k in range(offs[s] + max(fast - 1, 0), offs[s] + fast + 1):  # the segments at the fast vertex
+            assert np.array_equal(lists[k], here[np.abs(here - k) > 2])
+    for nc_x, lists_x in got[1:]:
+        assert np.array_equal(nc, nc_x)
+        for a, b in zip(lists, lists_x):
+            assert np.array_equal(a, b)

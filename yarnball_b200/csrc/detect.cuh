@@ -44,12 +44,14 @@ __device__ __forceinline__ Box<R> segment_box(const Dev<R>& d, int k, const Scen
 }
 
 // The same box in single precision, rounded outwards (exact in the FP32 build); one that is not
-// a number meets nothing.  The w components are free.
+// a number is empty.  lo.w holds an id (-1: no segment), hi.w is free.  The empty box meets a box that is
+// unbounded on every axis (a segment whose predicted displacement overflows has one), so a test against a
+// box that may be a placeholder looks at the id too.
 __device__ __forceinline__ float box_down(float x) { return x; }
 __device__ __forceinline__ float box_up(float x) { return x; }
 __device__ __forceinline__ float box_down(double x) { return __double2float_rd(x); }
 __device__ __forceinline__ float box_up(double x) { return __double2float_ru(x); }
-__device__ __forceinline__ float4 empty_lo() { return make_float4(INFINITY, INFINITY, INFINITY, 0.f); }
+__device__ __forceinline__ float4 empty_lo() { return make_float4(INFINITY, INFINITY, INFINITY, __int_as_float(-1)); }
 __device__ __forceinline__ float4 empty_hi() { return make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f); }
 
 __device__ __forceinline__ bool boxes_meet(const float4& alo, const float4& ahi, const float4& blo, const float4& bhi) {

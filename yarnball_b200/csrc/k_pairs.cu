@@ -194,7 +194,9 @@ __global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constan
     // clusters i and j >= i
     auto cross = [&](int j, const float4& blo, const float4& bhi) {
         const float4 vlo = d.lvlLo[0][base0 + j], vhi = d.lvlHi[0][base0 + j];
-        const bool ha = boxes_meet(alo, ahi, vlo, vhi), hb = boxes_meet(blo, bhi, ulo, uhi);
+        // the places past a scene's last segment hold none, whatever the boxes say
+        const bool ha = __float_as_int(alo.w) >= 0 && boxes_meet(alo, ahi, vlo, vhi);
+        const bool hb = __float_as_int(blo.w) >= 0 && boxes_meet(blo, bhi, ulo, uhi);
         const unsigned ma = __ballot_sync(FULL, ha), mb = __ballot_sync(FULL, hb);
         if (!ma || !mb) return;
         unsigned hits;
