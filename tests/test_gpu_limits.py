@@ -5,6 +5,9 @@ a box without bounds and an infinite filter distance, so it is listed with every
 scene that is no neighbour of it, and with nothing else: not with the vertices that start no
 segment, and not with the places past a scene's last segment in a cluster of 32.  The lists of all
 broadphase paths are the same.
+
+Configured again: a simulation of the same topology gets a fresh device state with all its segments:
+boxes, contacts and states are bit for bit those of one configured once.
 """
 import numpy as np
 import pytest
@@ -80,3 +83,35 @@ def test_unbounded_boxes_meet_segments_only(name, fast):
         assert np.array_equal(nc, nc_x)
         for a, b in zip(lists, lists_x):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("small_path", [True, False])
+def test_configured_again(small_path):
+    def fresh():
+        sim = _straight_yarns([[60, 60, 20]], 4)
+        sim.vels[:] = 0
+        sim.vels[:60, 1] = 0.3  # the first yarn towards the second
+        return sim
+
+    once, again = fresh(), fresh()
+    for s in (once, again):
+        s.set_small_path(small_path)
+    again.configure()
+    once.upload()
+    again.upload()
+    for s in (once, again):
+        s.setKBend(1e-8)
+        s.setKStretch(2e-2)
+    # configure() scales masses and rest rotors of the present ones: give both the same
+    for name in ("verts", "qs", "qRests"):
+        getattr(again, name)[...] = getattr(once, name)
+    for s in (once, again):
+        s.upload()
+    assert np.isfinite(np.concatenate(again.bounds())).all()  # before any detection
+    for s in (once, again):
+        s.advance(8 * H)
+    assert _lists(once)[0].sum() > 0
+    assert np.array_equal(_lists(once)[0], _lists(again)[0])
+    assert np.array_equal(np.concatenate(once.bounds()), np.concatenate(again.bounds()))
+    for a, b in zip(once.read_state_f64(), again.read_state_f64()):
+        assert np.array_equal(a, b)

@@ -470,6 +470,7 @@ struct Engine : EngineBase {
             YB_CUDA(cudaMemcpyAsync(d.wideAll, &kAll, sizeof(int), cudaMemcpyHostToDevice, S->stream));
         }
         YB_CUDA(upload_layout());
+        YB_CUDA(upload_clusters());  // no segments yet: every scene's table is empty, for bounds()
         launch_bvh_reset(d, S->stream);
         YB_CUDA(cudaStreamSynchronize(S->stream));
         return YB_OK;
@@ -1389,6 +1390,7 @@ yb_status yb_configure(yb_sim* S, float density) {
         delete S->eng;
         S->eng = nullptr;
         S->configured = false;
+        S->segs.clear();  // the new device state holds no segments yet: the upload below writes them
     }
     if (!S->ownStream) {
         cudaError_t e = cudaStreamCreateWithFlags(&S->ownStream, cudaStreamNonBlocking);
