@@ -376,6 +376,16 @@ yb_status yb_debug_last_vel(yb_sim* sim, double* lastVel3);
  * capacity partner ids into cols. */
 yb_status yb_debug_packed_contacts(yb_sim* sim, uint32_t* offsets, int32_t* cols, int64_t capacity);
 
+/* The Newton kernel that the next substep launches: 0 a shape with lanes per vertex (yb_set_tuning), 1 one
+ * warp owns 32 slots (small simulations), 2 and 3 32 slots with 256 and 128 threads, 4 and 5 128 slots
+ * (launched plainly, or as a programmatic dependent), 6 every contact evaluated without a test first (large
+ * simulations whose contacts were mostly in range in the last advance()); and how many contacts a
+ * vertex are staged on average (any pointer may be NULL).  States do not depend on either. */
+yb_status yb_debug_newton_kernel(yb_sim* sim, int32_t* kernel, int32_t* stagedPerVertex);
+/* Stages at most perVertex contacts a vertex on average, the rest are gathered (never more than were
+ * allocated; for tests of that path). */
+yb_status yb_debug_limit_staging(yb_sim* sim, int32_t perVertex);
+
 /* Runs only the substep phases selected by mask on the current device state:
  * 1 = predictor (initItr), 2 = detection with BVH rebuild, 4 = detection with refit only,
  * 8 = step limit, 16 = one Newton+orientation iteration, 32 = advection (endItr).

@@ -259,6 +259,31 @@ bool newton_may_take_all(const Dev<R>& d) {
     return sizeof(R) == 4 && d.n > 126 * 7 * d.sms;
 }
 
+// The load-balanced Newton kernel of a simulation's size and contacts (the reasons are at launch_iter).
+// The numbers are those of yb_debug_newton_kernel.
+enum NewtonKernel {
+    NEWTON_LANES = 0,      // k_iter: a shape with lanes per vertex was set
+    NEWTON_SMALL = 1,      // k_iter_small
+    NEWTON_32_WIDE = 2,    // k_iter_bal, 32 slots and 256 threads
+    NEWTON_32 = 3,         // k_iter_bal, 32 slots and 128 threads
+    NEWTON_128_PLAIN = 4,  // k_iter_bal, 128 slots, launched the plain way
+    NEWTON_128 = 5,        // k_iter_bal, 128 slots
+    NEWTON_ALL = 6         // k_iter_all
+};
+template <typename R>
+NewtonKernel newton_kernel(const Dev<R>& d) {
+    if constexpr (sizeof(R) == 4) {
+        if (d.n <= 30 * 2 * d.sms) return NEWTON_SMALL;
+        if (d.n <= 30 * 3 * d.sms) return NEWTON_32_WIDE;
+        if (d.n <= 30 * 6 * d.sms) return NEWTON_32;
+        if (!d.sift && newton_may_take_all(d)) return NEWTON_ALL;
+        return d.n <= 126 * 6 * d.sms ? NEWTON_128_PLAIN : NEWTON_128;
+    } else {
+        if (d.n <= 30 * d.sms) return NEWTON_SMALL;
+        return d.n <= 30 * 3 * d.sms ? NEWTON_32 : NEWTON_128_PLAIN;
+    }
+}
+
 // --- kernel launchers (stream-ordered; no host synchronisation) ---
 // clearLists: a detection follows; the contact counts are zeroed for it.
 template <typename R> void launch_init(const Dev<R>& d, bool clearLists, cudaStream_t s);

@@ -1029,42 +1029,47 @@ void launch_iter(const Dev<R>& d, int srcBuf, int threads, int lanes, int pipe, 
 #define YB_ITER(NT, T, MINB, P) \
     k_iter<R, NT, T, MINB, P><<<(d.n + (NT / T) - 3) / ((NT / T) - 2), NT, 0, s>>>(d, srcBuf)
     if (lanes == 0) {
-        // Load-balanced kernels.  A block of 128 slots fills the chip from about 112k vertices on (6
-        // blocks of 126 vertices on 148 SMs).  Below, a launch lasts as long as one block's chain
-        // of steps, so small blocks of 32 slots get 3 or 7 warps that only help with the contacts,
-        // while the grid still is one wave.  Time of 8 launches, 128 slots against 32 slots with
-        // 256 (128) threads: 91 against 69 (69) us at 1,949 vertices, 62 against 38 (43) at
-        // 12,827, 285 against 342 (283) at 65,792, 171 against 358 (228) at 100,352.  FP64 build,
-        // 32 slots with 128 threads against 128 slots: 69 against 103 us at 1,949 vertices, 102
-        // against 153 at 12,827, 503 against 383 at 94,560.
+        // Load-balanced kernels, chosen by newton_kernel().  A block of 128 slots fills the chip from about
+        // 112k vertices on (6 blocks of 126 vertices on 148 SMs).  Below, a launch lasts as long as one
+        // block's chain of steps, so small blocks of 32 slots get 3 or 7 warps that only help with the
+        // contacts, while the grid still is one wave.  Us per substep of whole advances, 32 slots with
+        // 128 threads / with 256 / 128 slots: swatches of 13,580, 19,400 and 25,220 vertices 116 / 134 / 152,
+        // 136 / 156 / 197 and 141 / 165 / 212, piles of 14,000 and 26,000 173 / 187 / 261 and 231 / 248 / 305.
+        // (Past a wave it would still gain for a while: 141 against 216 at 29,100, 174 against 232 at 48,500, 235
+        // against 235 at 77,600; the line does not use that yet.)  8 launches, 256 threads against 128: 69
+        // and 69 us at 1,949, 38 and 43 at 12,827.  FP64 build, 32 slots with 128 threads against 128 slots:
+        // 147 / 186 us a substep at 13,580, 215 / 269 at 29,100, 294 / 296 at 48,500.
         // k_iter_small wins while its blocks, two to an SM (FP64: one) for their registers, are one
         // wave; past that its second wave costs more: 6.9 against 9.7 us an iteration at 11,875
         // vertices, FP64 8.0 against 11.1 at 7,900.  The results are the same bit for bit.
-        // A grid that is most of one wave is launched the plain way: set up while the one before
-        // runs, its blocks would land on the SMs with the most room left instead of evenly (285
-        // against 315 us at 65,792 vertices).  Elsewhere the early set-up gains: 67 -> 59 us at
-        // 1,949, 103 -> 91 us FP64 at 12,827, 842 -> 827 us at 1.0M.
+        // A grid of 128 slots of at most one wave is launched the plain way: set up while the one before
+        // runs, its blocks would land on the SMs with the most room left instead of evenly.  Us per substep,
+        // plain / dependent: 216 / 228 at 29,100, 232 / 247 at 48,500, 237 / 261 at 77,600, pile of 105,000 753 /
+        // 748.  Elsewhere the early set-up gains: 67 -> 59 us at 1,949, 842 -> 827 us at 1.0M.  The FP64
+        // build has the plain way throughout: 238 / 246 at 19,400, 269 / 285 at 29,100, 296 / 298 at 48,500, pile of
+        // 200,000 1320 / 1317, of 1.0M 5897 / 5877.
         const size_t small = (d.n + 29) / 30, large = (d.n + 125) / 126;
-        if constexpr (sizeof(R) == 4) {
-            if (d.n <= 30 * 2 * d.sms)
-                launch_dependent(k_iter_small<R, 256, 2>, small, 256, s, d, srcBuf);
-            else if (d.n <= 30 * 3 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 256, 3>, small, 256, s, d, srcBuf);
-            else if (d.n <= 30 * 6 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 128, 6>, small, 128, s, d, srcBuf);
-            else if (!d.sift && newton_may_take_all(d))
-                launch_dependent(k_iter_all<R, 128, 7>, large, 128, s, d, srcBuf);
-            else if (d.n <= 126 * 6 * d.sms)
-                k_iter_bal<R, 128, 128, 6><<<large, 128, 0, s>>>(d, srcBuf);
-            else
-                launch_dependent(k_iter_bal<R, 128, 128, 6>, large, 128, s, d, srcBuf);
-        } else {
-            if (d.n <= 30 * d.sms)
-                launch_dependent(k_iter_small<R, 256, 1>, small, 256, s, d, srcBuf);
-            else if (d.n <= 30 * 3 * d.sms)
-                launch_dependent(k_iter_bal<R, 32, 128, 3>, small, 128, s, d, srcBuf);
-            else
-                k_iter_bal<R, 128, 128, 3><<<large, 128, 0, s>>>(d, srcBuf);
+        constexpr bool F32 = sizeof(R) == 4;
+        switch (newton_kernel(d)) {
+            case NEWTON_SMALL:
+                launch_dependent(k_iter_small<R, 256, F32 ? 2 : 1>, small, 256, s, d, srcBuf);
+                break;
+            case NEWTON_32_WIDE:
+                if constexpr (F32) launch_dependent(k_iter_bal<R, 32, 256, 3>, small, 256, s, d, srcBuf);
+                break;
+            case NEWTON_32:
+                launch_dependent(k_iter_bal<R, 32, 128, F32 ? 6 : 3>, small, 128, s, d, srcBuf);
+                break;
+            case NEWTON_128_PLAIN:
+                k_iter_bal<R, 128, 128, F32 ? 6 : 3><<<large, 128, 0, s>>>(d, srcBuf);
+                break;
+            case NEWTON_128:
+                if constexpr (F32) launch_dependent(k_iter_bal<R, 128, 128, 6>, large, 128, s, d, srcBuf);
+                break;
+            case NEWTON_ALL:
+                if constexpr (F32) launch_dependent(k_iter_all<R, 128, 7>, large, 128, s, d, srcBuf);
+                break;
+            case NEWTON_LANES: break;
         }
     } else if (pipe) {
         if (lanes == 4) YB_ITER(256, 4, 2, true);

@@ -401,6 +401,18 @@ class Sim:
                                                  int(off[-1])), "packed")
         return off, cols[:int(off[-1])]
 
+    NEWTON_KERNELS = ["k_iter", "k_iter_small", "k_iter_bal<32,256>", "k_iter_bal<32,128>", "k_iter_bal<128> plain",
+                      "k_iter_bal<128>", "k_iter_all"]
+
+    def debug_newton_kernel(self):
+        """(name of the Newton kernel of the next substep, contacts staged per vertex on average)."""
+        k, st = ctypes.c_int32(), ctypes.c_int32()
+        check(self._lib.yb_debug_newton_kernel(self._h, ctypes.byref(k), ctypes.byref(st)), "newton_kernel")
+        return self.NEWTON_KERNELS[k.value], st.value
+
+    def debug_limit_staging(self, perVertex):
+        check(self._lib.yb_debug_limit_staging(self._h, int(perVertex)), "limit_staging")
+
     def debug_last_vel(self):
         lv = np.zeros((self.numVerts, 3))
         check(self._lib.yb_debug_last_vel(self._h, ptr(lv, ctypes.c_double)), "lastVel")
