@@ -106,3 +106,40 @@ def test_staged_contacts_are_not_observable(n, precision):
     for other in states[1:]:
         for a, b in zip(states[0], other):
             assert np.array_equal(a, b)
+
+
+def _long_crossings(count, length, seed):
+    """`count` scenes of two yarns of two segments each, `length` metres long against a barrier reach of
+    1 mm, crossing at a small angle with a gap close to the reach."""
+    rng = np.random.default_rng(seed)
+    sim = Sim(scenes=[6] * count)
+    x = np.zeros((count, 2, 3, 3))
+    x[:, 0, :, 0] = (np.arange(3) - 1) * length
+    angle = np.exp(rng.uniform(np.log(0.01), np.log(0.2), count))
+    t = (np.arange(3) - 1)[None, :] * length - rng.uniform(-0.9, 0.9, (count, 1)) * length
+    x[:, 1, :, 0] = -rng.uniform(0.1, 0.9, (count, 1)) * length + t * np.cos(angle)[:, None]
+    x[:, 1, :, 1] = t * np.sin(angle)[:, None]
+    x[:, 1, :, 2] = rng.uniform(0.99e-3, 1.03e-3, (count, 1))
+    for s in range(count):
+        scenes.fill_yarns(sim, x[s].reshape(-1, 3).astype(np.float32), np.array([3, 3], np.int32), offset=6 * s,
+                          pin_first=False)
+    sim.set_meta_all(**dict(scenes.PILE_META, kCollision=1e-5))
+    sim.configure(1e-9)
+    sim.setKBend(1e-8)
+    sim.setKStretch(2e-2)
+    sim.maxH = 1e-3
+    sim.upload()
+    return sim
+
+
+@pytest.mark.parametrize("length", [0.02, 2.0, 20.0, 60.0])
+def test_contacts_of_long_segments_are_not_skipped(length):
+    """The bound that leaves contacts out holds however long the segments are against the barrier's reach:
+    the states are those of evaluating every contact (which is what happens with none staged)."""
+    sims = [_long_crossings(1500, length, 5) for _ in range(2)]
+    sims[1].debug_limit_staging(0)
+    for s in sims:
+        s.advance(H)
+    assert sims[0].debug_contacts()[0].sum() > 1500
+    for a, b in zip(sims[0].read_state_f64(), sims[1].read_state_f64()):
+        assert np.array_equal(a, b)

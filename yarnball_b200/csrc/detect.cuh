@@ -154,7 +154,11 @@ __device__ __forceinline__ R contact_step_limit(const Dev<R>& d, int k, size_t s
     const V3<R> nrm = xsub(xscale(uv.u, a1), xmix(b0, b1, uv.v));
     const R l = E::sqrt(xlen2(nrm));
     if (stage != NO_STAGE && d.relD) {
-        const R room = l - sp.outOfRange;
+        // The computed distance can lie above the true one by the rounding of the closest point's
+        // parameter, 3 roundings of |b| over the sine of the angle: 5.7e-6 |b| in single precision (below a
+        // sine of 0.03 the parameter is formed in FP64), 1e-8 |b| in double.  So does the Newton kernel's.
+        const R b = (fabs(b0.x) + fabs(b0.y) + fabs(b0.z)) + (fabs(b1.x) + fabs(b1.y) + fabs(b1.z));
+        const R room = l - (sp.outOfRange + R(sizeof(R) == 4 ? 2e-5 : 1e-7) * b);
         d.relD[stage] = room > R(0) ? room * room : R(-1);
     }
     pen = o > k && l <= sp.twoR;

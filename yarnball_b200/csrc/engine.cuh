@@ -99,7 +99,7 @@ struct SceneParams {
     R D;                            // damping / h
     R accel;                        // accelerationRatio
     R twoR;                         // 2 * radius
-    R outOfRange;                   // a contact farther apart than this has a gap above 1, with a margin for rounding
+    R outOfRange;                   // a contact farther apart than this has a gap above 1, with a margin for the gap's rounding
     R invb;                         // 1 / barrierThickness
     R kCol;                         // kCollision / barrierThickness
     R fricK, fricMu;                // kFriction, frictionCoeff

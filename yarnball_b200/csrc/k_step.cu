@@ -262,8 +262,8 @@ __global__ void __launch_bounds__(NT, MINB) k_iter(Dev<R> d, int src) {
 //     hold every pair within the detection radius); such a contact contributes exactly zero.
 //     No point pair of two segments can be closer than their distance at the start of the
 //     substep (from the list pass) less the largest relative displacement of their end points,
-//     so a contact with dist - max |dx_a - dx_b| > 2 radius + barrierThickness needs no
-//     closest points.  The bound is nearly tight, since neighbours move together: 56 % of the
+//     so a contact with dist - max |dx_a - dx_b| > 2 radius + barrierThickness, by a margin for the
+//     rounding of the distances (contact_step_limit), needs no closest points.  The bound is nearly tight, since neighbours move together: 56 % of the
 //     entries certified where 59 % are out of range (pile of 65,536 vertices, 12.4 contacts a
 //     segment), 59 of 65 % (uneven batch after 3 frames), 99 of 99 % (bundle of parallel yarns);
 //   * the others, queued in order, are evaluated NT at a time, one per thread; contributions go
