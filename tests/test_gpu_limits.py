@@ -12,6 +12,7 @@ boxes, contacts and states are bit for bit those of one configured once.
 import numpy as np
 import pytest
 
+import oracle
 from yarnball_b200 import scenes
 from yarnball_b200.sim import Sim
 
@@ -115,3 +116,37 @@ def test_configured_again(small_path):
     assert np.array_equal(np.concatenate(once.bounds()), np.concatenate(again.bounds()))
     for a, b in zip(once.read_state_f64(), again.read_state_f64()):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("small_path", [True, False])
+def test_opposite_contact_forces_cancel_before_the_own_terms(small_path):
+    """A yarn between two others that cross it at the same place: their forces on it are opposite and 10^5
+    times its weight.  Contacts are summed first, so they cancel exactly and the weight keeps its bits; with
+    the weight first, some 0.3 % of it would be rounded away.  One substep of one iteration against the
+    FP64 oracle; what is left is some twenty roundings of 6e-8, the bar is 1e-5."""
+    sim = Sim(18)
+    line = (np.arange(6) - 2.5) * 2e-3
+    x = np.zeros((3, 6, 3), np.float32)
+    x[0, :, 1], x[0, :, 2] = line, 0.5e-3
+    x[1, :, 0] = line
+    x[2, :, 1], x[2, :, 2] = line, -0.5e-3
+    scenes.fill_yarns(sim, x.reshape(-1, 3), np.array([6, 6, 6], np.int32), pin_first=False)
+    sim.verts["invMass"][:6] = 0
+    sim.verts["invMass"][12:] = 0
+    for k, v in dict(scenes.PILE_META, kCollision=1e-2, numItr=1).items():
+        setattr(sim.meta, k, v)
+    sim.meta.gravity = (0.0, 0.0, -9.8)
+    sim.configure()
+    sim.setKBend(1e-8)
+    sim.setKStretch(2e-2)
+    sim.maxH = H
+    sim.upload()
+    sim.set_small_path(small_path)
+    orc = oracle.from_sim(sim, mode=oracle.FP64)
+    sim.advance(H)
+    orc.advance(H, float(np.float32(H)))
+    got, ref = sim.read_state_f64()[0][8, 2], orc.state()["pos"][8, 2]
+    assert ref < -1e-12 and abs(got - ref) <= 1e-5 * abs(ref)
+    assert {2, 14} <= set(_lists(sim)[1][8].tolist())
+    sim.close()
+    orc.close()

@@ -12,8 +12,9 @@
 // shortened and split over roles:
 //   * `vt` vertex threads (one vertex each) and CT contact threads.  In a Newton iteration the
 //     contact threads evaluate the contacts, CT at a time and one per thread, while the vertex
-//     threads evaluate inertia, glue and stretch, then sum the contributions in list order and
-//     solve, beside the bending gradients of the contact threads; the next iteration's contacts
+//     threads evaluate inertia, glue and stretch, then sum the contributions in list order, add the own
+//     terms (after the contacts, so that large opposite contact forces cancel first: 1 % slower than
+//     before them) and solve, beside the bending gradients of the contact threads; the next iteration's contacts
 //     start as soon as the new displacements are known, beside the orientation update;
 //   * the pair search tests all padded boxes, every pair of vertices once, spread over all
 //     threads; hits go through a queue per warp so that the exact narrow phase runs on 32 pairs
@@ -300,12 +301,13 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
             R sl = own.sl;
             Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
             V3<R> dx(R(0));
+            OwnSums<R> mine{V3<R>(R(0)), V3<R>(R(0)), R(0), R(0)};
             if (chunks) evaluate(0, buf);
             if (valid) {
                 const D2<R> ad = DX[k];
                 dx = xyz(ad.a);
                 q0 = qof(QO[k]);
-                add_own_terms(d, own, DX, d.sp[sc].D, p0, e, dx, xyz(ad.b), q0, fa, Ha, fb, Hb);
+                mine = own_sums(d, own, DX, d.sp[sc].D, p0, e, dx, xyz(ad.b), q0);
             }
             for (int c = 0; c < max(chunks, 1); c++, buf ^= 1) {
                 // chunk c is evaluated, chunk c - 1 summed, and the rotors are those of the last iteration
@@ -333,6 +335,12 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                     }
                 }
             }
+            // own terms after the contacts, as in the multi-block kernels: large opposite contact forces
+            // cancel first
+            fa += mine.fa;
+            fb += mine.fb;
+            Ha.add_diag(mine.ha);
+            Hb.add_diag(mine.hb);
             V3<R> dxn = dx;
             if (vertexWarp) {
                 m.halo[0][k] = fb.x; m.halo[1][k] = fb.y; m.halo[2][k] = fb.z;

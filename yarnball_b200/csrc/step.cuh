@@ -325,33 +325,41 @@ __device__ __forceinline__ OwnTerms<R> own_terms(const Dev<R>& d, int k, const S
     return w;
 }
 
-// The vertex's own terms added to force and Hessian sums that already hold its contacts: inertia
-// (H = m/h^2, f = m/h^2 (y - dx)), the glue spring to a connected vertex, and the stretch-shear
-// coupling of segment k to its orientation (its other endpoint's share in fb, Hb).
+// The vertex's own terms of one iteration: inertia (H = m/h^2, f = m/h^2 (y - dx)), the glue spring to
+// a connected vertex, and the stretch-shear coupling of segment k to its orientation (its other
+// endpoint's share in fb, hb).  Their Hessians are multiples ha, hb of the identity.
 template <typename R>
-__device__ __forceinline__ void add_own_terms(const Dev<R>& d, const OwnTerms<R>& w, const D2<R>* __restrict__ DX, R D,
-                                              const V3<R>& p0, const V3<R>& e, const V3<R>& dx, const V3<R>& dx1,
-                                              const Q<R>& q0, V3<R>& fa, H3<R>& Ha, V3<R>& fb, H3<R>& Hb) {
+struct OwnSums {
+    V3<R> fa, fb;
+    R ha, hb;
+};
+
+template <typename R>
+__device__ __forceinline__ OwnSums<R> own_sums(const Dev<R>& d, const OwnTerms<R>& w, const D2<R>* __restrict__ DX, R D,
+                                               const V3<R>& p0, const V3<R>& e, const V3<R>& dx, const V3<R>& dx1,
+                                               const Q<R>& q0) {
+    OwnSums<R> o{V3<R>(R(0)), V3<R>(R(0)), R(0), R(0)};
     if (w.invMass != R(0)) {
-        Ha.add_diag(w.inertia);
-        fa += w.inertia * (w.y - dx);
+        o.ha = w.inertia;
+        o.fa = w.inertia * (w.y - dx);
     }
     if (w.cid >= 0) {
         const R stiff = R(40);
         const V3<R> pc = xyz(d.pos[w.cid]);
         const V3<R> dc = xyz(DX[w.cid].a);
-        fa -= stiff * ((p0 - pc) + (dx - dc) + D * dx);
-        Ha.add_diag(stiff * (R(1) + D));
+        o.fa -= stiff * ((p0 - pc) + (dx - dc) + D * dx);
+        o.ha += stiff * (R(1) + D);
     }
     if (w.flags & F_HAS_NEXT) {
         const V3<R> c = (e + (dx1 - dx)) * w.invl - qrotate(q0, V3<R>(R(1), R(0), R(0)));
         R dd = w.ks * w.invl;
-        fa += w.ks * c - (D * dd) * dx;
-        fb += -w.ks * c - (D * dd) * dx1;
+        o.fa += w.ks * c - (D * dd) * dx;
+        o.fb += -w.ks * c - (D * dd) * dx1;
         dd *= R(1) + D;
-        Ha.add_diag(dd);
-        Hb.add_diag(dd);
+        o.ha += dd;
+        o.hb += dd;
     }
+    return o;
 }
 
 // Whether segment k's orientation is updated, and the gradient b of its bending terms from the
