@@ -8,11 +8,14 @@ broadphase paths are the same.
 
 Configured again: a simulation of the same topology gets a fresh device state with all its segments:
 boxes, contacts and states are bit for bit those of one configured once.
+
+bounds(): the box of all padded segment boxes in the build's precision, rounded to the nearest float.
 """
 import numpy as np
 import pytest
 
 import oracle
+from tests.test_gpu_edges import _walks
 from yarnball_b200 import scenes
 from yarnball_b200.sim import Sim
 
@@ -150,3 +153,25 @@ def test_opposite_contact_forces_cancel_before_the_own_terms(small_path):
     assert {2, 14} <= set(_lists(sim)[1][8].tolist())
     sim.close()
     orc.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("traversal", [0, 2])
+def test_bounds_are_the_nearest_floats(precision, traversal):
+    R = np.float32 if precision == "fp32" else np.float64
+    for seed in range(6):
+        sim = _walks([60, 60, 37], seed, 0.02, precision=precision)
+        sim.set_small_path(False)
+        sim.set_traversal(traversal)
+        sim.debug_phases(1 | 2, H)
+        x, dx = sim.read_state_f64()[0].astype(R), sim.debug_dx().astype(R)
+        reach = np.sqrt(((dx * dx)[:, 0] + (dx * dx)[:, 1]) + (dx * dx)[:, 2])
+        reach = np.maximum(reach[:-1], reach[1:])
+        m = sim.meta
+        pad = (R(m.radius) + R(0.5) * R(m.barrierThickness)) * R(m.detectionScaler) + reach
+        seg = (sim.verts["flags"][:-1] & 2) != 0
+        lo = (np.minimum(x[:-1], x[1:]) - pad[:, None])[seg].min(0)
+        hi = (np.maximum(x[:-1], x[1:]) + pad[:, None])[seg].max(0)
+        got = sim.bounds()
+        assert np.array_equal(got[0], lo.astype(np.float32)) and np.array_equal(got[1], hi.astype(np.float32))
+        sim.close()

@@ -67,6 +67,26 @@ __device__ __forceinline__ void float_box(const Box<R>& b, float4& lo, float4& h
     }
 }
 
+// The same box rounded to nearest, for the union that bounds() reports; a test of it widens it by one
+// float on each side (in the FP32 build it is exact and stays).
+template <typename R>
+__device__ __forceinline__ void nearest_box(const Box<R>& b, float4& lo, float4& hi) {
+    lo = make_float4((float)b.mn[0], (float)b.mn[1], (float)b.mn[2], 0.f);
+    hi = make_float4((float)b.mx[0], (float)b.mx[1], (float)b.mx[2], 0.f);
+    if (!(lo.x <= hi.x && lo.y <= hi.y && lo.z <= hi.z)) {
+        lo = empty_lo();
+        hi = empty_hi();
+    }
+}
+template <typename R>
+__device__ __forceinline__ void widen_box(float4& lo, float4& hi) {
+    if constexpr (sizeof(R) == 8) {
+        const float tiny = __uint_as_float(1u);  // the smallest float: the directed sum is the next one
+        lo.x = __fadd_rd(lo.x, -tiny); lo.y = __fadd_rd(lo.y, -tiny); lo.z = __fadd_rd(lo.z, -tiny);
+        hi.x = __fadd_ru(hi.x, tiny); hi.y = __fadd_ru(hi.y, tiny); hi.z = __fadd_ru(hi.z, tiny);
+    }
+}
+
 // Narrow-phase decision for segments x < y (both with hasNext, same scene): not joined by a
 // connection, not neighbours on a yarn, and closer than the filter distance, to which each
 // segment adds its reach.

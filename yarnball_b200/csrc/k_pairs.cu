@@ -21,8 +21,9 @@
 // in 269 scenes, 3.2 contacts a segment: 1.27 + 3.9 ms -> 0.17 + 2.2 ms; one pile of 65,792
 // vertices, 11.5 contacts: 49 + 280 us -> 10 + 75 us; a swatch of 1,949 vertices: 32 + 78 us -> 7 + 12 us.
 //
-// Boxes are kept in single precision in both builds, rounded outwards in the FP64 one: a box
-// may only be too large, and what it lets through the filter decides.
+// Boxes are kept in single precision in both builds: in the FP64 one segments' boxes are rounded
+// outwards, and those of nodes to nearest (bounds() reports their union) and widened by a float where
+// they are tested.  A tested box may only be too large, and what it lets through the filter decides.
 #include "detect.cuh"
 
 namespace yb {
@@ -64,18 +65,22 @@ __global__ void __launch_bounds__(BOX_THREADS) k_boxes(Dev<R> d, const int* __re
     float4 lo = empty_lo(), hi = empty_hi();
     if (c < sc.count[0]) {
         const int p = 32 * c + lane;
-        int k = -1;
+        const size_t at = 32 * (size_t)(sc.lvl[0] + c) + lane;
         if (p < sc.segCount) {
-            k = sortedVals[sc.segBase + p];
+            const int k = sortedVals[sc.segBase + p];
             R reach;
             const Box<R> b = segment_box(d, k, d.sp[s], reach);
-            float_box(b, lo, hi);
-            hi.w = (float)reach;
+            float4 slo, shi;
+            float_box(b, slo, shi);
+            slo.w = __int_as_float(k);
+            shi.w = (float)reach;
+            d.leafLo[at] = slo;
+            d.leafHi[at] = shi;
+            nearest_box(b, lo, hi);
+        } else {
+            d.leafLo[at] = empty_lo();
+            d.leafHi[at] = empty_hi();
         }
-        const size_t at = 32 * (size_t)(sc.lvl[0] + c) + lane;
-        lo.w = __int_as_float(k);
-        d.leafLo[at] = lo;
-        d.leafHi[at] = hi;
         warp_box(lo, hi);
         if (lane == 0) {
             d.lvlLo[0][sc.lvl[0] + c] = lo;
@@ -180,7 +185,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constan
     const int base0 = sc.lvl[0], top = sc.top;
     const int i = ci - base0;
     const float4 alo = d.leafLo[32 * (size_t)ci + lane], ahi = d.leafHi[32 * (size_t)ci + lane];
-    const float4 ulo = d.lvlLo[0][ci], uhi = d.lvlHi[0][ci];
+    float4 ulo = d.lvlLo[0][ci], uhi = d.lvlHi[0][ci];
+    widen_box<R>(ulo, uhi);
     int qn = 0;  // queued pairs (identical in every lane)
 
     // lanes (own box, own segment) against the r boxes packed in sh.lo / sh.hi
@@ -193,7 +199,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constan
     };
     // clusters i and j >= i
     auto cross = [&](int j, const float4& blo, const float4& bhi) {
-        const float4 vlo = d.lvlLo[0][base0 + j], vhi = d.lvlHi[0][base0 + j];
+        float4 vlo = d.lvlLo[0][base0 + j], vhi = d.lvlHi[0][base0 + j];
+        widen_box<R>(vlo, vhi);
         // the places past a scene's last segment hold none, whatever the boxes say
         const bool ha = __float_as_int(alo.w) >= 0 && boxes_meet(alo, ahi, vlo, vhi);
         const bool hb = __float_as_int(blo.w) >= 0 && boxes_meet(blo, bhi, ulo, uhi);
@@ -256,8 +263,11 @@ __global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constan
     auto meet = [&](int level, int base) {
         const int at = base + lane;
         bool hit = false;
-        if (at < sc.count[level] && at >= (i >> (5 * level)))
-            hit = boxes_meet(d.lvlLo[level][sc.lvl[level] + at], d.lvlHi[level][sc.lvl[level] + at], ulo, uhi);
+        if (at < sc.count[level] && at >= (i >> (5 * level))) {
+            float4 lo = d.lvlLo[level][sc.lvl[level] + at], hi = d.lvlHi[level][sc.lvl[level] + at];
+            widen_box<R>(lo, hi);
+            hit = boxes_meet(lo, hi, ulo, uhi);
+        }
         return __ballot_sync(FULL, hit);
     };
 
