@@ -143,3 +143,42 @@ def test_contacts_of_long_segments_are_not_skipped(length):
     assert sims[0].debug_contacts()[0].sum() > 1500
     for a, b in zip(sims[0].read_state_f64(), sims[1].read_state_f64()):
         assert np.array_equal(a, b)
+
+
+def _yarns(n):
+    sim = Sim(n)
+    x = np.zeros((n, 3), np.float32)
+    x[:, 0] = np.arange(n) % 250 * 2e-3
+    x[:, 1] = np.arange(n) // 250 * 5e-3
+    scenes.fill_yarns(sim, x, np.full(n // 250, 250, np.int32), pin_first=True)
+    for k, v in scenes.PILE_META.items():
+        setattr(sim.meta, k, v)
+    return sim
+
+
+def test_staged_contacts_follow_the_size_and_what_fits():
+    """The number of staged contacts is a rule of the simulation's size, whatever else is on the device; where
+    that many do not fit, 7 or 1 are taken, and the states are the same bit for bit."""
+    import torch
+
+    n = 1000000
+    sim = _ready(_yarns(n))
+    assert sim.debug_newton_kernel()[1] == 16
+    sim.advance(2 * H)
+    state = sim.read_state_f64()
+    size = {16: sim.device_bytes()}
+    sim.close()
+    for slots in (7, 1):
+        size[slots] = size[16] - (16 - slots) * 28 * n
+    room = {16: 2 * size[16], 7: (size[7] + size[16]) // 2, 1: (size[1] + size[7]) // 2}
+    for slots, free in room.items():
+        torch.cuda.empty_cache()
+        held = torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+        sim = _ready(_yarns(n))
+        assert sim.debug_newton_kernel()[1] == slots
+        del held
+        torch.cuda.empty_cache()
+        sim.advance(2 * H)
+        for a, b in zip(state, sim.read_state_f64()):
+            assert np.array_equal(a, b)
+        sim.close()

@@ -68,8 +68,10 @@ struct alignas(sizeof(R) * 2) R2 {
 
 // Staged contacts: RELCAP x vertices slots in all; a contact past them is gathered and never certified
 // out of range (with 8 the Newton launches of a bundle with 13.7 contacts a segment take 370 us
-// instead of 171).  Simulations of more than an eighth of the free device memory have RELCAP_LARGE.
+// instead of 171).  Simulations of more than LARGE_BYTES of device memory (an eighth of a B200's) have
+// RELCAP_LARGE: a rule of the size alone, so that a simulation runs alike whatever else is on the device.
 constexpr int RELCAP = 16, RELCAP_LARGE = 7;
+constexpr size_t LARGE_BYTES = 22ull << 30;
 constexpr int LIST_THREADS = 128;  // vertices per block of the list pass (one packed-offset tile)
 constexpr int SMALL_TILE = 32;     // ... in a small simulation
 __host__ __device__ constexpr int list_tiles(int n) { return (n + SMALL_TILE - 1) / SMALL_TILE; }  // at most

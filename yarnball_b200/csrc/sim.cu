@@ -416,16 +416,15 @@ struct Engine : EngineBase {
             relSlots = slots;
             return sum;
         };
-        // A simulation that takes much of the device stages fewer contacts (the rest are gathered), and one
-        // that would not fit stages hardly any.
-        size_t freeBytes = 0, deviceBytes = 0;
-        YB_CUDA(cudaMemGetInfo(&freeBytes, &deviceBytes));
+        // A large simulation stages fewer contacts (the rest are gathered), and so does one that would not
+        // fit otherwise.
         off = total(RELCAP);
-        if (off > freeBytes / 8) off = total(RELCAP_LARGE);
+        if (off > LARGE_BYTES) off = total(RELCAP_LARGE);
         cudaError_t got = cudaMalloc(&block, off);
-        if (got == cudaErrorMemoryAllocation) {
+        for (size_t fewer : {(size_t)RELCAP_LARGE, (size_t)1}) {
+            if (got != cudaErrorMemoryAllocation || fewer >= relSlots) continue;
             cudaGetLastError();
-            off = total(1);
+            off = total(fewer);
             got = cudaMalloc(&block, off);
         }
         YB_CUDA(got);
