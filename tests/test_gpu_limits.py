@@ -9,6 +9,9 @@ broadphase paths are the same.
 Configured again: a simulation of the same topology gets a fresh device state with all its segments:
 boxes, contacts and states are bit for bit those of one configured once.
 
+Walks over the BVH: its memory is taken when one of them is first chosen; where it does not fit the call
+says so, the mode stays, and the simulation goes on.
+
 bounds(): the box of all padded segment boxes in the build's precision, rounded to the nearest float.
 """
 import numpy as np
@@ -175,3 +178,42 @@ def test_bounds_are_the_nearest_floats(precision, traversal):
         got = sim.bounds()
         assert np.array_equal(got[0], lo.astype(np.float32)) and np.array_equal(got[1], hi.astype(np.float32))
         sim.close()
+
+
+def test_bvh_memory_is_taken_with_the_first_walk():
+    import torch
+
+    from yarnball_b200._abi import YarnBallError
+
+    n = 200000
+    sims = []
+    for _ in range(2):
+        sim = _walks([250] * (n // 250), 3, 0.12)
+        sims.append(sim)
+        plain = sim.device_bytes()
+        assert plain < 2000 * n
+    sims[0].set_traversal(0)
+    assert sims[0].device_bytes() >= plain + 250 * n
+    sims[0].set_traversal(1)  # no second one
+    assert sims[0].device_bytes() < plain + 260 * n
+    sims[0].advance(2 * H)
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(YarnBallError):
+        sims[1].set_traversal(0)
+    del held
+    torch.cuda.empty_cache()
+    assert sims[1].device_bytes() == plain
+    sims[1].advance(2 * H)
+    for a, b in zip(sims[0].read_state_f64(), sims[1].read_state_f64()):
+        assert np.array_equal(a, b)
+    sims[1].set_traversal(0)
+    for s in sims:
+        s.set_traversal(2)
+        s.advance(H)
+        s.set_traversal(0)
+        s.advance(H)
+    for a, b in zip(sims[0].read_state_f64(), sims[1].read_state_f64()):
+        assert np.array_equal(a, b)
+    for s in sims:
+        s.close()

@@ -37,7 +37,7 @@ __global__ void k_scene_box_init(Dev<R> d) {
         d.sceneBox[6 * s + a] = 0xFFFFFFFFu;
         d.sceneBox[6 * s + 3 + a] = 0u;
     }
-    d.sceneRoot[s] = INT_MIN;
+    if (d.sceneRoot) d.sceneRoot[s] = INT_MIN;  // (null while there is no BVH)
 }
 
 // Per-scene bounds of segment midpoints (Morton normalisation).

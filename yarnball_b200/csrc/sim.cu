@@ -66,7 +66,7 @@ struct EngineBase {
     virtual yb_status drive_pins(double dt) = 0;
     virtual yb_status residual_substep(int type, double* out, int cap, int* count) = 0;
     virtual yb_status read_last_vel(double* out) = 0;
-    virtual void set_traversal(int packet) = 0;
+    virtual yb_status set_traversal(int packet) = 0;
     virtual bool small_fits() const = 0;
     virtual yb_status run_small(int steps) = 0;
     virtual yb_status packed_contacts(uint32_t* off, int32_t* cols, int64_t capacity) = 0;
@@ -324,6 +324,7 @@ struct Engine : EngineBase {
         for (auto& g : graphs)
             if (g) cudaGraphExecDestroy(g);
         if (block) cudaFree(block);
+        if (bvhMem) cudaFree(bvhMem);
         if (pinMem) cudaFree(pinMem);
         if (spHost) cudaFreeHost(spHost);
         if (errHost) cudaFreeHost(errHost);
@@ -335,7 +336,6 @@ struct Engine : EngineBase {
     yb_status alloc() {
         const size_t n = (size_t)S->capVerts;
         const size_t ns = (size_t)S->capScenes;
-        const size_t nn = n > 1 ? n - 1 : 1;
         sortBytes = radix_sort_scratch_bytes((int)n);
         size_t off = 0;
         std::vector<std::pair<void**, size_t>> req;
@@ -367,21 +367,6 @@ struct Engine : EngineBase {
         want((void**)&d.segs, sizeof(int) * n);
         want((void**)&spDev, sizeof(SceneParams<R>) * ns);
         want((void**)&d.err, sizeof(int) * EW_COUNT);
-        want((void**)&d.nodes, sizeof(BNode<R>) * nn);
-        want((void**)&d.wide, sizeof(WNode<R>) * nn);
-        want((void**)&d.depJump[0], sizeof(int) * nn);
-        want((void**)&d.depJump[1], sizeof(int) * nn);
-        want((void**)&d.depDist[0], sizeof(int) * nn);
-        want((void**)&d.depDist[1], sizeof(int) * nn);
-        want((void**)&d.wideUsed, nn);
-        want((void**)&d.wideAll, sizeof(int));
-        want((void**)&d.qrec, sizeof(QRec<R>) * n);
-        want((void**)&d.nodeLast, sizeof(int) * nn);
-        want((void**)&d.leafParent, sizeof(int) * n);
-        want((void**)&d.refitCount, sizeof(unsigned) * nn);
-        want((void**)&d.sceneRoot, sizeof(int) * ns);
-        want((void**)&d.sceneLast, sizeof(int) * ns);
-        want((void**)&d.travNext, sizeof(unsigned) * 4);
         // clusters: the last one of a scene may be partly filled, and so may the last node of a level
         size_t nodesCap[CLUS_LEVELS];
         for (int l = 0; l < CLUS_LEVELS; l++) nodesCap[l] = (l ? nodesCap[l - 1] : n) / 32 + ns;
@@ -460,9 +445,45 @@ struct Engine : EngineBase {
         // no packed contacts until the first list pass (a Newton launch before it reads none)
         YB_CUDA(cudaMemsetAsync(d.csrOff, 0, sizeof(unsigned) * (n + 1), S->stream));
         YB_CUDA(cudaMemsetAsync(d.lastVel, 0, sizeof(V4<R>) * n, S->stream));
-        YB_CUDA(cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * nn, S->stream));
         for (int l = 0; l < CLUS_LEVELS; l++)
             YB_CUDA(cudaMemsetAsync(d.lvlCount[l], 0, sizeof(unsigned) * nodesCap[l], S->stream));
+        YB_CUDA(upload_layout());
+        YB_CUDA(upload_clusters());  // no segments yet: every scene's table is empty, for bounds()
+        YB_CUDA(cudaStreamSynchronize(S->stream));
+        return d.travPacket == 2 ? YB_OK : alloc_bvh();
+    }
+
+    // The BVH of the walks (yb_set_traversal 0 and 1), 253 bytes a vertex, allocated when they are
+    // first chosen.
+    void* bvhMem = nullptr;
+    yb_status alloc_bvh() {
+        if (bvhMem) return YB_OK;
+        const size_t n = (size_t)S->capVerts, nn = n > 1 ? n - 1 : 1, ns = (size_t)S->capScenes;
+        const std::pair<void**, size_t> req[] = {
+            {(void**)&d.nodes, sizeof(BNode<R>) * nn},   {(void**)&d.wide, sizeof(WNode<R>) * nn},
+            {(void**)&d.depJump[0], sizeof(int) * nn},   {(void**)&d.depJump[1], sizeof(int) * nn},
+            {(void**)&d.depDist[0], sizeof(int) * nn},   {(void**)&d.depDist[1], sizeof(int) * nn},
+            {(void**)&d.wideUsed, nn},                   {(void**)&d.wideAll, sizeof(int)},
+            {(void**)&d.qrec, sizeof(QRec<R>) * n},      {(void**)&d.nodeLast, sizeof(int) * nn},
+            {(void**)&d.leafParent, sizeof(int) * n},    {(void**)&d.refitCount, sizeof(unsigned) * nn},
+            {(void**)&d.sceneRoot, sizeof(int) * ns},    {(void**)&d.sceneLast, sizeof(int) * ns},
+            {(void**)&d.travNext, sizeof(unsigned) * 4},
+        };
+        size_t bytes = 0;
+        for (auto& r : req) bytes += (r.second + 255) & ~(size_t)255;
+        const cudaError_t got = cudaMalloc(&bvhMem, bytes);
+        if (got != cudaSuccess) {
+            cudaGetLastError();
+            bvhMem = nullptr;
+            return cuda_status(got);
+        }
+        allocBytes += bytes;
+        size_t off = 0;
+        for (auto& r : req) {
+            *r.first = (char*)bvhMem + off;
+            off += (r.second + 255) & ~(size_t)255;
+        }
+        YB_CUDA(cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * nn, S->stream));
         // records never built read as empty (last = 0 prunes every entry); until the first
         // rebuild marks the nodes, every record is built
         YB_CUDA(cudaMemsetAsync(d.wide, 0, sizeof(WNode<R>) * nn, S->stream));
@@ -470,8 +491,6 @@ struct Engine : EngineBase {
             static const int kAll = 1;
             YB_CUDA(cudaMemcpyAsync(d.wideAll, &kAll, sizeof(int), cudaMemcpyHostToDevice, S->stream));
         }
-        YB_CUDA(upload_layout());
-        YB_CUDA(upload_clusters());  // no segments yet: every scene's table is empty, for bounds()
         launch_bvh_reset(d, S->stream);
         YB_CUDA(cudaStreamSynchronize(S->stream));
         return YB_OK;
@@ -989,14 +1008,19 @@ struct Engine : EngineBase {
         return YB_OK;
     }
 
-    void set_traversal(int packet) override {
-        if (d.travPacket == packet) return;
+    yb_status set_traversal(int packet) override {
+        if (d.travPacket == packet) return YB_OK;
+        if (packet != 2) {
+            const yb_status st = alloc_bvh();
+            if (st != YB_OK) return st;
+        }
         invalidate_graphs();
         if ((d.travPacket == 2) != (packet == 2)) {  // the BVH is kept by the BVH walks only
             bvhBuilt = false;
             S->lastBVHRebuild = INFINITY;
         }
         d.travPacket = packet;
+        return YB_OK;
     }
 
     yb_status read_last_vel(double* out) override {
@@ -1664,8 +1688,11 @@ yb_status yb_set_small_path(yb_sim* S, int32_t enable) {
 
 yb_status yb_set_traversal(yb_sim* S, int32_t packet) {
     if (!S || packet < 0 || packet > 2) return YB_ERR_INVALID_ARGUMENT;
+    if (S->eng) {
+        const yb_status st = S->eng->set_traversal(packet);
+        if (st != YB_OK) return st;  // the BVH does not fit: the mode stays
+    }
     S->travPacket = packet;
-    if (S->eng) S->eng->set_traversal(packet);
     return YB_OK;
 }
 
@@ -1979,8 +2006,8 @@ yb_status yb_batch_gather(int32_t count, yb_sim* const* srcSims, const int32_t* 
         }
         S->configured = true;
     }
-    S->eng->set_traversal(S->travPacket);
-    yb_status st = S->eng->gather(count, srcSims, srcScenes);
+    yb_status st = S->eng->set_traversal(S->travPacket);
+    if (st == YB_OK) st = S->eng->gather(count, srcSims, srcScenes);
     if (st == YB_OK) st = validate_all_meta(S);
     if (st == YB_OK) S->eng->write_params();
     if (st != YB_OK) {
