@@ -16,8 +16,8 @@
 //                   (the broadphase appends here; the list pass sorts each row)
 //   csrOff   u32    n + 1: the contacts of vertex k, packed in vertex order by the list pass
 //                   every substep, are slots [csrOff[k], csrOff[k+1]) of
-//   csrCols  int    partner ids (sorted within each vertex's range)
-//   csrOwner u8     low byte of the vertex each packed contact belongs to
+//   csrCols  u32    packed contacts (sorted within each vertex's range): partner id and, above it,
+//                   the low byte of the vertex the contact belongs to
 //   relA/B/D V4,R2,R  partner endpoints relative to p0 and the squared room to the barrier's reach,
 //                   staged per substep in the same slots while the slot is below relCap
 // Segments are the vertices with hasNext; segs[] lists them, scene after scene.
@@ -82,6 +82,15 @@ __host__ __device__ constexpr int list_tiles(int n) { return (n + SMALL_TILE - 1
 // deeper tree gets every record.
 constexpr int DEPTH_ROUNDS = 7;
 constexpr int DEPTH_LAUNCHES = 1 + DEPTH_ROUNDS + 1;  // init, jumps, marks
+
+// A packed contact: the partner's id (a simulation has at most 2^31 / MAX_COLS = 2^24 vertices) and the low
+// byte of its owner, so that a Newton block reads both at once.
+static_assert((1ll << 31) / MAX_COLS <= 1ll << 24, "partner ids have 24 bits");
+__device__ __forceinline__ unsigned packed_contact(int partner, int owner) {
+    return (unsigned)partner | (unsigned)owner << 24;
+}
+__host__ __device__ __forceinline__ int packed_partner(unsigned e) { return (int)(e & 0xffffffu); }
+__device__ __forceinline__ int packed_owner(unsigned e) { return (int)(e >> 24); }
 
 // Contact-list addressing: each segment owns a row of MAX_COLS partner ids.
 __host__ __device__ __forceinline__ size_t col_at(int seg, int c) { return (size_t)seg * MAX_COLS + c; }
@@ -184,8 +193,7 @@ struct Dev {
     R* relD;          //   squared room: how far the centre lines are beyond the barrier's reach at the
                       //   start of the substep, -1 when they are not (null: not kept)
     unsigned* csrOff; // n + 1 packed offsets (see the layout above)
-    int* csrCols;     // csrCap packed partner ids
-    unsigned char* csrOwner;  // low byte of each packed contact's vertex
+    unsigned* csrCols;  // csrCap packed contacts
     unsigned csrCap;  // slots of csrCols
     unsigned relCap;  // slots of relA / relB
     unsigned long long* listStatus;  // list pass: [0] tile ticket, [1 + tile] look-back status;

@@ -803,10 +803,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
             }
             const int s = slot, ks = tile * B + s;
             const unsigned long long g = base + (unsigned long long)f;
-            if (g < (unsigned long long)d.csrCap) {
-                d.csrCols[g] = o;
-                d.csrOwner[g] = (unsigned char)ks;
-            }
+            if (g < (unsigned long long)d.csrCap) d.csrCols[g] = packed_contact(o, ks);
             const V3<R> oa0(sA0[0][s], sA0[1][s], sA0[2][s]);
             const V3<R> oa1(sA1[0][s], sA1[1][s], sA1[2][s]);
             bool pen = false;

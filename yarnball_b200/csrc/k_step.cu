@@ -137,11 +137,11 @@ __global__ void __launch_bounds__(NT, MINB) k_iter(Dev<R> d, int src) {
             // registers); without it each contact loads then computes.
             unsigned off;
             const int nc = contact_range(d, k, off);
-            const int* __restrict__ cl = d.csrCols + off;
+            const unsigned* __restrict__ cl = d.csrCols + off;
             const V3<R> e = p1 - p0;
             if constexpr (!PIPE) {
                 for (int c2 = lane; c2 < nc; c2 += T) {
-                    const int j = __ldg(cl + c2);
+                    const int j = packed_partner(__ldg(cl + c2));
                     if (!partner_ok(d, j)) continue;
                     V3<R> r0, r1;
                     partner_rel(d, off + c2, j, p0, r0, r1);
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter(Dev<R> d, int src) {
             D2<R> pdn;
             bool okn = false;
             if (c2 < nc) {
-                const int j = __ldg(cl + c2);
+                const int j = packed_partner(__ldg(cl + c2));
                 okn = partner_ok(d, j);
                 if (okn) {
                     partner_rel(d, off + c2, j, p0, r0n, r1n);
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter(Dev<R> d, int src) {
                 const bool ok = okn;
                 c2 += T;
                 if (c2 < nc) {
-                    const int j = __ldg(cl + c2);
+                    const int j = packed_partner(__ldg(cl + c2));
                     okn = partner_ok(d, j);
                     if (okn) {
                         partner_rel(d, off + c2, j, p0, r0n, r1n);
@@ -360,8 +360,9 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
                 j2 = -1;
                 if (f < fEnd) {
                     const unsigned g = base + (unsigned)f;
-                    j2 = __ldg(d.csrCols + g);
-                    s2 = (int)__ldg(d.csrOwner + g);
+                    const unsigned e = __ldg(d.csrCols + g);
+                    j2 = packed_partner(e);
+                    s2 = packed_owner(e);
                     room2 = g < d.relCap ? d.relD[g] : R(-1);
                     if (!partner_ok(d, j2)) j2 = -1;
                 }
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_bal(Dev<R> d, int src) {
                 if (t == 0 || queued(i - 1) >> 16 != s) sFirst[s] = (short)t;
                 if (t == NT - 1 || i + 1 == lives || queued(i + 1) >> 16 != s) sEnd[s] = (short)(t + 1);
                 const unsigned g = base + (unsigned)(e & 0xffff);
-                const int j = __ldg(d.csrCols + g);
+                const int j = packed_partner(__ldg(d.csrCols + g));
                 const D2<R> pd = DX[j];
                 const V4<R> A = sA[s], Bq = sB[s];
                 V3<R> r0, r1;
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
     // The partner id of this thread's contact is loaded one chunk ahead (after the previous
     // chunk's barrier, before its summation), so a chunk starts with the partner gather.
     int jn = 0;
-    if (t < total) jn = __ldg(d.csrCols + (base + t));
+    if (t < total) jn = packed_partner(__ldg(d.csrCols + (base + t)));
     for (int b0 = 0; b0 < total; b0 += NT, buf ^= 1) {
         const int f = b0 + t;
         {
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
             const int fn = b0 + NT + t;
             if (fn < total) {
                 const unsigned g = base + fn;
-                jn = __ldg(d.csrCols + g);
+                jn = packed_partner(__ldg(d.csrCols + g));
                 if (g < d.relCap) {
                     prefetch_l1(d.relA + g);
                     prefetch_l1(d.relB + g);
@@ -816,8 +817,9 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_small(Dev<R> d, int src) {
             const unsigned g = base + (unsigned)f;
             j[q] = -1;
             if (f < fEnd && g < d.csrCap) {
-                j[q] = __ldg(d.csrCols + g);
-                s[q] = ((int)__ldg(d.csrOwner + g) - kb) & 31;
+                const unsigned e = __ldg(d.csrCols + g);
+                j[q] = packed_partner(e);
+                s[q] = (packed_owner(e) - kb) & 31;
                 room[q] = g < d.relCap ? d.relD[g] : R(-1);
             }
         }
@@ -921,7 +923,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_small(Dev<R> d, int src) {
                 if (h == 0 || queued(i - 1) >> 16 != so) sFirst[so] = (short)h;
                 if (h == HELP - 1 || i + 1 == lives || queued(i + 1) >> 16 != so) sEnd[so] = (short)(h + 1);
                 const unsigned g = base + (unsigned)(en & 0xffff);
-                const int jo = __ldg(d.csrCols + g);
+                const int jo = packed_partner(__ldg(d.csrCols + g));
                 const D2<R> po = DX[jo];
                 const V4<R> A = sA[so], Bq = sB[so];
                 V3<R> r0, r1;

@@ -361,8 +361,7 @@ struct Engine : EngineBase {
         const size_t csrCap = std::min(n * (size_t)MAX_COLS, (size_t)0xffffffffu);
         const size_t listTiles = (size_t)list_tiles((int)n);
         want((void**)&d.csrOff, sizeof(unsigned) * (n + 1));
-        want((void**)&d.csrCols, sizeof(int) * csrCap);
-        want((void**)&d.csrOwner, csrCap);
+        want((void**)&d.csrCols, sizeof(unsigned) * csrCap);
         want((void**)&d.listStatus, sizeof(unsigned long long) * (1 + listTiles));
         want((void**)&d.segs, sizeof(int) * n);
         want((void**)&spDev, sizeof(SceneParams<R>) * ns);
@@ -1048,6 +1047,7 @@ struct Engine : EngineBase {
         if (cols && total) {
             YB_CUDA(cudaMemcpyAsync(cols, d.csrCols, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st));
             YB_CUDA(cudaStreamSynchronize(st));
+            for (size_t i = 0; i < total; i++) cols[i] = packed_partner((uint32_t)cols[i]);
         }
         return YB_OK;
     }
