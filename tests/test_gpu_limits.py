@@ -12,6 +12,9 @@ boxes, contacts and states are bit for bit those of one configured once.
 Walks over the BVH: its memory is taken when one of them is first chosen; where it does not fit the call
 says so, the mode stays, and the simulation goes on.
 
+A scene of more than 2^20 segments, whose clusters have a third level above them: the lists of the walk over
+the BVH, and the same states.
+
 bounds(): the box of all padded segment boxes in the build's precision, rounded to the nearest float.
 """
 import numpy as np
@@ -19,6 +22,7 @@ import pytest
 
 import oracle
 from tests.test_gpu_edges import _walks
+from tests.test_gpu_newton import _pairs_of_yarns
 from yarnball_b200 import scenes
 from yarnball_b200.sim import Sim
 
@@ -217,3 +221,23 @@ def test_bvh_memory_is_taken_with_the_first_walk():
         assert np.array_equal(a, b)
     for s in sims:
         s.close()
+
+
+def test_clusters_of_more_than_a_million_segments():
+    states, lists = [], []
+    for mode in (0, 2):
+        sim = _pairs_of_yarns(2110, 250)
+        assert ((sim.verts["flags"] & 2) != 0).sum() > 1 << 20
+        sim.set_traversal(mode)
+        for mask in (1 | 2, 4):  # a rebuilt order, then the same refitted
+            sim.debug_phases(mask, H if mask & 1 else 0.0)
+            lists.append(sim.debug_packed_contacts())
+        sim.advance(2 * H)
+        lists.append(sim.debug_packed_contacts())
+        states.append(sim.read_state_f64() + sim.bounds())
+        sim.close()
+    for (off, cols), (off2, cols2) in zip(lists[:3], lists[3:]):
+        assert off[-1] > 1 << 20
+        assert np.array_equal(off, off2) and np.array_equal(cols, cols2)
+    for a, b in zip(*states):
+        assert np.array_equal(a, b)
