@@ -311,7 +311,8 @@ template <typename R> void reset_list_status(const Dev<R>& d, cudaStream_t s);
 // Segment, cluster and level boxes in curve order; the cluster-pair search; per-scene boxes.
 template <typename R> void launch_boxes(const Dev<R>& d, cudaStream_t s);
 template <typename R> void launch_pairs(const Dev<R>& d, cudaStream_t s);
-template <typename R> void launch_scene_box(const Dev<R>& d, float* out, cudaStream_t s);
+template <typename R> void launch_cluster_box(const Dev<R>& d, float* out, cudaStream_t s);
+template <typename R> void launch_scene_box(const Dev<R>& d, float* out, cudaStream_t s);  // of the walk in use
 template <typename R> void launch_bvh_reset(const Dev<R>& d, cudaStream_t s);
 // Places driven vertices on their prescribed motion at the start of an advance of length dt.
 template <typename R>

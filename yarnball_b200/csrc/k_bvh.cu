@@ -40,7 +40,7 @@ __global__ void k_scene_box_init(Dev<R> d) {
     if (d.sceneRoot) d.sceneRoot[s] = INT_MIN;  // (null while there is no BVH)
 }
 
-// Per-scene bounds of segment midpoints (Morton normalisation).
+// Per-scene bounds of segment midpoints, for the cells of the curve.
 template <typename R>
 __global__ void __launch_bounds__(256) k_scene_bounds(Dev<R> d) {
     const int si = blockIdx.x * blockDim.x + threadIdx.x;
@@ -357,7 +357,7 @@ constexpr int TRAV_QCAP = 160;      // < 32 left over + up to 4 candidates per l
 constexpr int TRAV_GRAB = 32;       // queries a warp takes from the counter at a time
 
 // Broadphase + narrow phase.  Every segment queries the tree once with its own box (the
-// sorted leaves of the last rebuild, taken in Morton order, so neighbouring lanes start on
+// sorted leaves of the last rebuild, taken in curve order, so neighbouring lanes start on
 // neighbouring queries).  Each unordered pair is found by exactly one of its two segments:
 // the one with the lower sorted position, whose walk skips every entry holding only leaves at
 // or before its own position.  The walk runs over the wide nodes (four grandchildren per
@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(NT) k_lists(Dev<R> d, int sortLists) {
 }
 
 // Packet traversal: a warp walks the tree once for 32 consecutive queries (consecutive sorted
-// positions, so neighbouring segments in Morton order).  Every lane tests its own box against
+// positions, so neighbouring segments in curve order).  Every lane tests its own box against
 // the entries of the node the warp has loaded (one record, read by all lanes at the same
 // address); the warp descends into an internal entry when any of its lanes overlaps it, keeping
 // one stack per warp in shared memory.  The walk is the union of the 32 walks of k_traverse,
@@ -995,6 +995,36 @@ void launch_bvh_rebuild(const Dev<R>& d, cudaStream_t s, void* sortScratch, size
     launch_bvh_refit(d, s);
 }
 
+// Box of each scene while the walks keep the BVH: that of its subtree's root (k_refit must have run).
+template <typename R>
+__global__ void k_scene_root_box(Dev<R> d, float* out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= d.numScenes) return;
+    const int r = d.sceneRoot[s];
+    float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    if (r >= 0) {
+        const BNode<R>& nd = d.nodes[r];
+        for (int a = 0; a < 3; a++) {
+            b[a] = (float)ymin(nd.lmin[a], nd.rmin[a]);
+            b[3 + a] = (float)ymax(nd.lmax[a], nd.rmax[a]);
+        }
+    } else if (r != INT_MIN) {  // a single segment
+        R reach;
+        const Box<R> bx = segment_box(d, -r - 1, d.sp[s], reach);
+        for (int a = 0; a < 3; a++) { b[a] = (float)bx.mn[a]; b[3 + a] = (float)bx.mx[a]; }
+    }
+    for (int a = 0; a < 6; a++) out[6 * s + a] = b[a];
+}
+
+template <typename R>
+void launch_scene_box(const Dev<R>& d, float* out, cudaStream_t s) {
+    if (d.numScenes <= 0) return;
+    if (d.travPacket == 2)
+        launch_cluster_box(d, out, s);
+    else
+        k_scene_root_box<R><<<(d.numScenes + 127) / 128, 128, 0, s>>>(d, out);
+}
+
 template <typename R>
 void launch_bvh_reset(const Dev<R>& d, cudaStream_t s) {
     if (d.numScenes > 0) k_scene_box_init<R><<<(d.numScenes + 127) / 128, 128, 0, s>>>(d);
@@ -1003,8 +1033,10 @@ void launch_bvh_reset(const Dev<R>& d, cudaStream_t s) {
 template <typename R>
 void launch_bvh_refit(const Dev<R>& d, cudaStream_t s) {
     if (d.nseg <= 0) return;
-    launch_boxes(d, s);  // by every walk, for bounds()
-    if (d.travPacket == 2) return;
+    if (d.travPacket == 2) {
+        launch_boxes(d, s);
+        return;
+    }
     // one segment: no internal node, but its query record is written
     if (d.nseg > 1) cudaMemsetAsync(d.refitCount, 0, sizeof(unsigned) * (d.nseg - 1), s);
     k_refit<R><<<(d.nseg + 255) / 256, 256, 0, s>>>(d, d.vals[0]);
@@ -1062,6 +1094,8 @@ template void launch_bvh_rebuild<float>(const Dev<float>&, cudaStream_t, void*, 
 template void launch_bvh_rebuild<double>(const Dev<double>&, cudaStream_t, void*, size_t, int);
 template void launch_bvh_refit<float>(const Dev<float>&, cudaStream_t);
 template void launch_bvh_refit<double>(const Dev<double>&, cudaStream_t);
+template void launch_scene_box<float>(const Dev<float>&, float*, cudaStream_t);
+template void launch_scene_box<double>(const Dev<double>&, float*, cudaStream_t);
 template void launch_bvh_reset<float>(const Dev<float>&, cudaStream_t);
 template void launch_bvh_reset<double>(const Dev<double>&, cudaStream_t);
 template <typename R>

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 32) k_pairs(const __grid_constan
     if (qn) pairs_filter(d, sh, 0, qn, s);
 }
 
-// Box of each scene: the union of its top level (at most 32 nodes; k_boxes must have run).
+// Box of each scene: the union of its clusters' top level (at most 32 nodes; k_boxes must have run).
 template <typename R>
 __global__ void __launch_bounds__(32) k_scene_box(Dev<R> d, float* out) {
     const SceneClus sc = d.sceneClus[blockIdx.x];
@@ -340,14 +340,14 @@ void launch_pairs(const Dev<R>& d, cudaStream_t s) {
 }
 
 template <typename R>
-void launch_scene_box(const Dev<R>& d, float* out, cudaStream_t s) {
-    if (d.numScenes > 0) k_scene_box<R><<<d.numScenes, 32, 0, s>>>(d, out);
+void launch_cluster_box(const Dev<R>& d, float* out, cudaStream_t s) {
+    k_scene_box<R><<<d.numScenes, 32, 0, s>>>(d, out);
 }
 
 #define YB_INST(R)                                               \
     template void launch_boxes<R>(const Dev<R>&, cudaStream_t);  \
     template void launch_pairs<R>(const Dev<R>&, cudaStream_t);  \
-    template void launch_scene_box<R>(const Dev<R>&, float*, cudaStream_t);
+    template void launch_cluster_box<R>(const Dev<R>&, float*, cudaStream_t);
 YB_INST(float)
 YB_INST(double)
 

@@ -490,7 +490,10 @@ struct Engine : EngineBase {
             static const int kAll = 1;
             YB_CUDA(cudaMemcpyAsync(d.wideAll, &kAll, sizeof(int), cudaMemcpyHostToDevice, S->stream));
         }
-        launch_bvh_reset(d, S->stream);
+        Dev<R> all = d;
+        all.numScenes = S->capScenes;  // a recycled batch may hold more later
+        launch_bvh_reset(all, S->stream);
+        YB_CUDA(cudaGetLastError());
         YB_CUDA(cudaStreamSynchronize(S->stream));
         return YB_OK;
     }
@@ -856,7 +859,7 @@ struct Engine : EngineBase {
     int num_itr() const { return (int)S->meta[0].numItr; }
 
     // Kernels of a rebuild and of a refit, with the boxes of either.
-    uint64_t refit_launches() const { return d.travPacket == 2 ? 1 : 3; }
+    uint64_t refit_launches() const { return d.travPacket == 2 ? 1 : 2; }
     uint64_t rebuild_launches() const {
         const int passes = d.nseg > 1 ? (keyBits + 7) / 8 : 0;
         return 3 + (d.nseg > 1 ? 2 + passes : 0) + (d.travPacket == 2 ? 0 : 1 + DEPTH_LAUNCHES) + refit_launches();
