@@ -637,10 +637,11 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
     for (int g = myOff; g < min(myOff + nc, NT); g++) sOwn[0][g] = t;
     __syncthreads();
     int buf = 0;
-    // The partner id of this thread's contact is loaded one chunk ahead (after the previous
-    // chunk's barrier, before its summation), so a chunk starts with the partner gather.
-    int jn = 0;
-    if (t < total) jn = packed_partner(__ldg(d.csrCols + (base + t)));
+    // The packed contact of this thread is loaded one chunk ahead (after the previous chunk's barrier,
+    // before its summation), so a chunk starts with the partner gather; it is unpacked there, since an
+    // operation on it here would wait for the load (+5 % on the whole kernel).
+    unsigned en = 0;
+    if (t < total) en = __ldg(d.csrCols + (base + t));
     for (int b0 = 0; b0 < total; b0 += NT, buf ^= 1) {
         const int f = b0 + t;
         {
@@ -651,9 +652,9 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
         V3<R> cfa(R(0)), cfb(R(0));
         H3<R> cHa, cHb;
         cHa.zero(); cHb.zero();
-        if (f < total && partner_ok(d, jn)) {
+        const int j = packed_partner(en);
+        if (f < total && partner_ok(d, j)) {
             const int s = sOwn[buf][t];
-            const int j = jn;
             const V3<R> sp0(sSeg[0][s], sSeg[1][s], sSeg[2][s]);
             V3<R> r0, r1;
             partner_rel(d, base + f, j, sp0, r0, r1);
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iter_all(Dev<R> d, int src) {
             const int fn = b0 + NT + t;
             if (fn < total) {
                 const unsigned g = base + fn;
-                jn = packed_partner(__ldg(d.csrCols + g));
+                en = __ldg(d.csrCols + g);
                 if (g < d.relCap) {
                     prefetch_l1(d.relA + g);
                     prefetch_l1(d.relB + g);
