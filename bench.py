@@ -80,7 +80,7 @@ def workload_desc(spec):
         "substeps_per_step": SUBSTEPS,
         "newton_iterations": NUM_ITR,
         "step": "advance(1/30 s) of the whole batch (%d substeps of h=1/%d s)" % (SUBSTEPS, SUBSTEPS * 30),
-        "l2": "inputs larger than L2 (one Newton iteration alone moves ~260 B of DRAM traffic per vertex, "
+        "l2": "inputs larger than L2 (one Newton iteration alone moves ~270 B of DRAM traffic per vertex, "
               "%.1f GB for %.1fM vertices, against 126 MB of L2), no flush" % (n * 260e-9, n / 1e6),
         "seed": SEED,
         "parallelism": "one GPU",
@@ -149,14 +149,18 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-def load_traffic():
-    """Per-vertex DRAM bytes of one Newton iteration from the committed ncu summary."""
+def load_traffic(kernel=None):
+    """DRAM bytes of one Newton launch from the committed ncu summaries: of `kernel` (a name of
+    `Sim.debug_newton_kernel`, None when it has no capture), or of the kernel that tests contacts first."""
     p = os.path.join(ROOT, "profiles", "k_iter_traffic.json")
     try:
         with open(p) as f:
-            return json.load(f)
+            tr = json.load(f)
     except Exception:
         return None
+    if kernel is None or kernel == tr["newton_kernel"]:
+        return tr
+    return tr["others"].get(kernel)
 
 
 def oracle_sample(spec, target_verts, mode, seed=SEED):
@@ -302,20 +306,25 @@ def run_ours(args):
     l0 = sim.launch_count()
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
+    newton_kernels = {}  # frames by the Newton kernel that they ran
     e0.record(stream)
     for _ in range(args.steps):
+        kernel = sim.debug_newton_kernel()[0]  # host state only
+        newton_kernels[kernel] = newton_kernels.get(kernel, 0) + 1
         sim.advance(FRAME)
     e1.record(stream)
     torch.cuda.synchronize()
     if dist:
         dist.barrier()
     ck = clocks.stop()
+    cfg["newton_kernels"] = newton_kernels
     launches = sim.launch_count() - l0
     ms = e0.elapsed_time(e1)
     ms_max, n_all = sharding.reduce_timing(ms, n, device="cuda")
     value = n_all * SUBSTEPS * args.steps / (ms_max / 1e3)
 
     # Per-kernel device times of one more frame (events around each kernel class).
+    newton_kernel = sim.debug_newton_kernel()[0]
     prof_ms, prof_launches = sim.profile_advance(FRAME)
     total_pairs, segs_with, max_cols = sim.collisionStats()
     nseg = int(((sim.verts["flags"] & 2) != 0).sum())
@@ -325,25 +334,19 @@ def run_ours(args):
     bytes_per_launch = n * (ITER_BYTES_BASE + ITER_BYTES_PER_CONTACT * cbar)
     achieved = bytes_per_launch / (iter_ms / 1e3) / 1e9
     peak, peak_kind = load_peaks()
-    tr = load_traffic()
+    tr = load_traffic(newton_kernel)
     traffic, traffic_src = None, None
-    if tr and tr.get("vertices") == n and tr.get("warmup") == args.warmup:
-        # captured on this workload at the first Newton launch of the timed region; the mean
-        # launch of the region has more contacts, so scale by the algorithmic bytes
+    if tr:
+        # a launch of the same kernel on this workload, scaled by the algorithmic bytes to the mean launch
+        # of the profiled frame (another contact count, or another state or size)
         traffic = tr["dram_bytes_per_launch"] * bytes_per_launch / tr["algorithmic_bytes_per_launch"]
-        traffic_src = ("ncu capture of the first Newton launch of this workload after %d warm-up frames "
-                       "(c = %.2f), scaled to the mean launch's algorithmic bytes (%s)") % (
-            tr["warmup"], tr["cbar_at_capture"], tr["summary"])
-    elif tr:
-        # another state or size: the captured traffic per algorithmic byte
-        traffic = tr["dram_bytes_per_launch"] * bytes_per_launch / tr["algorithmic_bytes_per_launch"]
-        traffic_src = "ncu capture (%d vertices, %d warm-up frames, c = %.2f) scaled by the algorithmic bytes (%s)" % (
-            tr["vertices"], tr["warmup"], tr["cbar_at_capture"], tr["summary"])
+        traffic_src = "ncu capture of %s (%d vertices, %d warm-up frames, c = %.2f) scaled by the algorithmic bytes (%s)" % (
+            newton_kernel, tr["vertices"], tr["warmup"], tr["cbar_at_capture"], tr["summary"])
     prof_total = sum(prof_ms.values())
     roofline = {
         "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
         "traffic": traffic, "traffic_source": traffic_src,
-        "kernel": "k_iter (fused Newton position solve + orientation update)",
+        "kernel": newton_kernel + " (fused Newton position solve + orientation update)",
         "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
         "algorithmic_bytes_per_launch": bytes_per_launch, "avg_launch_ms": iter_ms, "cbar": cbar,
         "kernel_share": {k: v / prof_total for k, v in prof_ms.items()},

@@ -35,3 +35,17 @@ def test_peak_is_measured_or_the_stated_fallback():
         assert kind == "measured" and peak > 0
     else:
         assert (peak, kind) == (6650.0, "fallback")
+
+
+def test_traffic_record_of_each_newton_kernel():
+    b = _bench()
+    first = b.load_traffic()
+    assert b.load_traffic("k_iter_bal<128>") == first
+    every = b.load_traffic("k_iter_all")
+    assert every["newton_kernel"] == "k_iter_all" and every["dram_bytes_per_launch"] != first["dram_bytes_per_launch"]
+    assert every["dram_bytes_per_launch"] == every["dram_bytes_read_per_launch"] + every["dram_bytes_write_per_launch"]
+    alg = every["vertices"] * (b.ITER_BYTES_BASE + b.ITER_BYTES_PER_CONTACT * every["cbar_at_capture"])
+    assert abs(alg - every["algorithmic_bytes_per_launch"]) / alg < 1e-3
+    assert os.path.exists(os.path.join(ROOT, every["summary"]))
+    # a kernel without a capture has no traffic figure rather than another kernel's
+    assert b.load_traffic("k_iter_small") is None
