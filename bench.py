@@ -81,7 +81,7 @@ def workload_desc(spec):
         "newton_iterations": NUM_ITR,
         "step": "advance(1/30 s) of the whole batch (%d substeps of h=1/%d s)" % (SUBSTEPS, SUBSTEPS * 30),
         "l2": "inputs larger than L2 (one Newton iteration alone moves ~270 B of DRAM traffic per vertex, "
-              "%.1f GB for %.1fM vertices, against 126 MB of L2), no flush" % (n * 260e-9, n / 1e6),
+              "%.1f GB for %.1fM vertices, against 126 MB of L2), no flush" % (n * 270e-9, n / 1e6),
         "seed": SEED,
         "parallelism": "one GPU",
     }
