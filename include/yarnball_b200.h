@@ -199,7 +199,9 @@ yb_status yb_autotune(yb_sim* sim, int32_t* bestThreads, int32_t* bestLanes, int
 
 /* Broadphase: packet = 2 (default) searches pairs of clusters of 32 segments that are
  * consecutive along a space-filling curve, a warp per cluster; packet = 1 walks a BVH once per
- * warp for 32 consecutive queries, packet = 0 once per query.  The contact lists are identical. */
+ * warp for 32 consecutive queries, packet = 0 once per query.  The contact lists are identical.
+ * The first choice of 0 or 1 allocates the BVH; where it does not fit, the mode stays and the error is
+ * returned. */
 yb_status yb_set_traversal(yb_sim* sim, int32_t packet);
 yb_status yb_get_traversal(yb_sim* sim, int32_t* packet);
 
