@@ -13,7 +13,7 @@
 //   * `vt` vertex threads (one vertex each) and CT contact threads.  In a Newton iteration the
 //     contact threads evaluate the contacts, CT at a time and one per thread, while the vertex
 //     threads evaluate inertia, glue and stretch, then sum the contributions in list order, add the own
-//     terms (after the contacts, so that large opposite contact forces cancel first: 1 % slower than
+//     terms (after the contacts, so that large opposite contact forces cancel first: up to 1 % slower than
 //     before them) and solve, beside the bending gradients of the contact threads; the next iteration's contacts
 //     start as soon as the new displacements are known, beside the orientation update;
 //   * the pair search tests all padded boxes, every pair of vertices once, spread over all
@@ -53,7 +53,7 @@ struct SmallShare {
     V4<R> relA[CAP];
     R2<R> relB[CAP];
     int pack[CAP];         // owner << 16 | partner
-    R halo[10][SMALL_VERTS];  // fb, Hb and the step limit of each segment
+    R halo[10][SMALL_VERTS];  // each vertex's own terms, then fb, Hb and the step limit of each segment
     V4<R> bend[SMALL_VERTS];  // gradient of each segment's bending terms
     float4 boxLo[SMALL_VERTS], boxHi[SMALL_VERTS];
     unsigned adj[SMALL_VERTS][SMALL_WORDS];
@@ -301,13 +301,20 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
             R sl = own.sl;
             Q<R> q0 = qmk(R(0), R(0), R(0), R(1));
             V3<R> dx(R(0));
-            OwnSums<R> mine{V3<R>(R(0)), V3<R>(R(0)), R(0), R(0)};
             if (chunks) evaluate(0, buf);
-            if (valid) {
-                const D2<R> ad = DX[k];
-                dx = xyz(ad.a);
-                q0 = qof(QO[k]);
-                mine = own_sums(d, own, DX, d.sp[sc].D, p0, e, dx, xyz(ad.b), q0);
+            // The own terms wait for the contacts in rows of the halo, which are free until then: in registers
+            // they make the FP64 build spill (216 vertices: 92 us a substep, 84 this way).
+            if (vertexWarp) {
+                OwnSums<R> mine{V3<R>(R(0)), V3<R>(R(0)), R(0), R(0)};
+                if (valid) {
+                    const D2<R> ad = DX[k];
+                    dx = xyz(ad.a);
+                    q0 = qof(QO[k]);
+                    mine = own_sums(d, own, DX, d.sp[sc].D, p0, e, dx, xyz(ad.b), q0);
+                }
+                m.halo[0][k] = mine.fa.x; m.halo[1][k] = mine.fa.y; m.halo[2][k] = mine.fa.z;
+                m.halo[3][k] = mine.fb.x; m.halo[4][k] = mine.fb.y; m.halo[5][k] = mine.fb.z;
+                m.halo[6][k] = mine.ha; m.halo[7][k] = mine.hb;
             }
             for (int c = 0; c < max(chunks, 1); c++, buf ^= 1) {
                 // chunk c is evaluated, chunk c - 1 summed, and the rotors are those of the last iteration
@@ -335,14 +342,14 @@ __global__ void __launch_bounds__(SMALL_VERTS + SmallShare<R>::CT)
                     }
                 }
             }
-            // own terms after the contacts, as in the multi-block kernels: large opposite contact forces
-            // cancel first
-            fa += mine.fa;
-            fb += mine.fb;
-            Ha.add_diag(mine.ha);
-            Hb.add_diag(mine.hb);
             V3<R> dxn = dx;
             if (vertexWarp) {
+                // own terms after the contacts, as in the multi-block kernels: large opposite contact forces
+                // cancel first
+                fa += V3<R>(m.halo[0][k], m.halo[1][k], m.halo[2][k]);
+                fb += V3<R>(m.halo[3][k], m.halo[4][k], m.halo[5][k]);
+                Ha.add_diag(m.halo[6][k]);
+                Hb.add_diag(m.halo[7][k]);
                 m.halo[0][k] = fb.x; m.halo[1][k] = fb.y; m.halo[2][k] = fb.z;
 #pragma unroll
                 for (int q = 0; q < 6; q++) m.halo[3 + q][k] = Hb.d[q];
